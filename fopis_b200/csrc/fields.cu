@@ -87,38 +87,61 @@ __global__ void convert_species_kernel(const W* rho, long long N, double scale, 
         out[t] = scale * weight_value(rho[t]);
 }
 
-// Glue copy of one axis: node 0 <- node n, node n+1 <- node 1
-// (Communicator::sendRecvFieldX/Y/Z self branch, Communicator.cpp:290-299).
-__global__ void glue_kernel(double* a, G g, int axis) {
+// Glue copies of every periodic axis at once: node 0 <- node n, node n+1 <-
+// node 1 (Communicator::sendRecvFieldX/Y/Z self branch, Communicator.cpp:290-299,
+// axis after axis): a glue node takes the node with all its periodic indices
+// wrapped, which no copy writes. Nodes on two planes are written twice, alike.
+struct Planes {
+    long long start[7];   // first item of each plane or face
+    int axis[6], side[6];
+    int n;
+};
+__global__ void glue_kernel(double* a, G g, Planes f) {
     const int dims[3] = {g.cx, g.cy, g.cz};
-    const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
-    const long long plane = (long long)dims[a1] * dims[a2];
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < plane; t += (long long)gridDim.x * blockDim.x) {
-        int idx[3];
-        idx[a1] = (int)(t / dims[a2]);
-        idx[a2] = (int)(t % dims[a2]);
-        const int X = dims[axis];
-        idx[axis] = 1; const double lo = a[L(g, idx[0], idx[1], idx[2])];
-        idx[axis] = X - 2; const double hi = a[L(g, idx[0], idx[1], idx[2])];
-        idx[axis] = 0; a[L(g, idx[0], idx[1], idx[2])] = hi;
-        idx[axis] = X - 1; a[L(g, idx[0], idx[1], idx[2])] = lo;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < f.start[f.n]; t += (long long)gridDim.x * blockDim.x) {
+        int q = 0;
+        while (t >= f.start[q + 1]) ++q;
+        const int axis = f.axis[q], a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
+        const int r = (int)(t - f.start[q]);
+        int idx[3], src[3];
+        idx[a1] = r / dims[a2];
+        idx[a2] = r % dims[a2];
+        idx[axis] = f.side[q] ? dims[axis] - 1 : 0;
+        for (int d = 0; d < 3; ++d) {
+            src[d] = idx[d];
+            if (g.per[2 * d]) src[d] = idx[d] == 0 ? dims[d] - 2 : (idx[d] == dims[d] - 1 ? 1 : idx[d]);
+        }
+        a[L(g, idx[0], idx[1], idx[2])] = a[L(g, src[0], src[1], src[2])];
     }
 }
 
-// Field::setDirichletPhi / setNeumannPhi on one face (src/Grid/Field.cpp:34-96):
-// the face plane over the interior of the other two axes.
-__global__ void phi_face_kernel(double* phi, G g, int axis, int side, int neumann) {
+// Field::setDirichletPhi / setNeumannPhi (src/Grid/Field.cpp:34-96) on every
+// face in one launch: the face planes over the interior of the other two axes,
+// in the reference's order x-, x+, y-, ... A node on several faces keeps the
+// last one's value: zero, or the node one step inwards as the faces before it
+// left that, so the walk goes down the axes; it ends off the faces, at nodes
+// that nothing here writes.
+__global__ void phi_face_kernel(double* phi, G g, Planes f, unsigned neumann) {
     const int dims[3] = {g.cx, g.cy, g.cz};
-    const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
-    const long long m1 = dims[a1] - 2, m2 = dims[a2] - 2;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < m1 * m2; t += (long long)gridDim.x * blockDim.x) {
-        int idx[3];
-        idx[a1] = 1 + (int)(t / m2);
-        idx[a2] = 1 + (int)(t % m2);
-        const int X = dims[axis];
-        const int bi = side == 0 ? 1 : X - 2, ni = side == 0 ? 2 : X - 3;
-        idx[axis] = ni; const double nv = phi[L(g, idx[0], idx[1], idx[2])];
-        idx[axis] = bi; phi[L(g, idx[0], idx[1], idx[2])] = neumann ? nv : 0.0;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < f.start[f.n]; t += (long long)gridDim.x * blockDim.x) {
+        int q = 0;
+        while (t >= f.start[q + 1]) ++q;
+        const int axis = f.axis[q], a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
+        const int r = (int)(t - f.start[q]), m2 = dims[a2] - 2;
+        int idx[3], src[3];
+        idx[a1] = 1 + r / m2;
+        idx[a2] = 1 + r % m2;
+        idx[axis] = f.side[q] ? dims[axis] - 2 : 1;
+        bool held = false;
+        for (int d = 2; d >= 0; --d) {
+            src[d] = idx[d];
+            if (held || g.per[2 * d]) continue;
+            const int hi = idx[d] == dims[d] - 2;
+            if (!hi && idx[d] != 1) continue;
+            if ((neumann >> (2 * d + hi)) & 1u) src[d] = hi ? dims[d] - 3 : 2;
+            else held = true;
+        }
+        phi[L(g, idx[0], idx[1], idx[2])] = held ? 0.0 : phi[L(g, src[0], src[1], src[2])];
     }
 }
 
@@ -231,15 +254,23 @@ void rho_zero(Ctx& c) {
     FOPIS_CUDA(cudaMemsetAsync(c.rho_i64, 0, sizeof(unsigned long long) * c.N * c.nsp, c.st));
 }
 
+static void add_plane(Planes& f, int axis, int side, long long items) {
+    f.axis[f.n] = axis;
+    f.side[f.n] = side;
+    f.start[f.n + 1] = f.start[f.n] + items;
+    ++f.n;
+}
+
 void glue_copy(Ctx& c, double* a) {
     const G g = make_g(c);
     const long long planes[3] = {(long long)c.cy * c.cz, (long long)c.cx * c.cz, (long long)c.cx * c.cy};
-    for (int axis = 0; axis < 3; ++axis) {
-        if (!c.per[2 * axis]) continue;
-        ++c.launches;
-        glue_kernel<<<blocks(planes[axis]), kT, 0, c.st>>>(a, g, axis);
-        FOPIS_LAUNCH_CHECK();
-    }
+    Planes f{};
+    for (int axis = 0; axis < 3; ++axis)
+        for (int side = 0; side < 2 && c.per[2 * axis]; ++side) add_plane(f, axis, side, planes[axis]);
+    if (f.n == 0) return;
+    ++c.launches;
+    glue_kernel<<<blocks(f.start[f.n]), kT, 0, c.st>>>(a, g, f);
+    FOPIS_LAUNCH_CHECK();
 }
 
 void rho_finalize(Ctx& c) {
@@ -275,16 +306,21 @@ void rho_finalize(Ctx& c) {
 void phi_boundary(Ctx& c) {
     const G g = make_g(c);
     glue_copy(c, c.phi);
+    Planes f{};
+    unsigned neumann = 0;
+    const long long m[3] = {(long long)(c.cy - 2) * (c.cz - 2), (long long)(c.cx - 2) * (c.cz - 2),
+                            (long long)(c.cx - 2) * (c.cy - 2)};
     for (int axis = 0; axis < 3; ++axis)
         for (int side = 0; side < 2; ++side) {
             const char b = c.p.boundary[2 * axis + side];
             if (b == 'P') continue;
-            const long long m = axis == 0 ? (long long)(c.cy - 2) * (c.cz - 2)
-                                          : (axis == 1 ? (long long)(c.cx - 2) * (c.cz - 2) : (long long)(c.cx - 2) * (c.cy - 2));
-            ++c.launches;
-            phi_face_kernel<<<blocks(m), kT, 0, c.st>>>(c.phi, g, axis, side, b == 'N');
-            FOPIS_LAUNCH_CHECK();
+            if (b == 'N') neumann |= 1u << (2 * axis + side);
+            add_plane(f, axis, side, m[axis]);
         }
+    if (f.n == 0) return;
+    ++c.launches;
+    phi_face_kernel<<<blocks(f.start[f.n]), kT, 0, c.st>>>(c.phi, g, f, neumann);
+    FOPIS_LAUNCH_CHECK();
 }
 
 void efield_update(Ctx& c) {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/fopis_gpu.h"
@@ -27,6 +28,25 @@ struct ApiError {
     int code;
     std::string msg;
 };
+
+// Launches a solver kernel, with the programmatic-serialization attribute when
+// pdl is set: its launch is then processed as the previous kernel's blocks
+// retire, and it waits (griddepcontrol.wait) before it touches memory.
+template <typename... KArgs, typename... Args>
+void launch_k(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+              Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    FOPIS_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+}
 
 // ------------------------------------------------------------------ packed cells
 // A particle's node cell (glue-layout indices i = floor(x)+1 ...) packed into
@@ -112,7 +132,7 @@ struct DevScalars {
     unsigned long long injected;
     unsigned long long not_found;
     unsigned int status;                                // FOPIS_DEV_* bits
-    unsigned int pad;
+    unsigned int ticket;                                // blocks of the running residual kernel that finished
     unsigned long long pointwise_bits;                  // last solve's pointwise residual (double bits)
     // per species in the current fused step: valid particles the push moved, those that
     // stayed valid (in the domain, not absorbed), and particles injected or emitted
@@ -179,6 +199,19 @@ struct MGLevel {
     float* r = nullptr;  // residual scratch
     double scale = 1.0;  // operator scale 1/4^level relative to the fine level
     size_t size() const { return (size_t)n[0] * n[1] * n[2]; }
+};
+
+// One axis of the fast-diagonalisation solve (direct.cu): n unknowns, np
+// mirrored pairs, he = n - np even modes (np odd ones), matrices padded to hp.
+struct DirectAxis {
+    int n = 0, per = 0, np = 0, he = 0, hp = 0;
+    const float *we = nullptr, *wo = nullptr;   // [folded index][mode], even and odd half
+    const float *te = nullptr, *to = nullptr;   // their transposes
+    const float* lam = nullptr;                 // eigenvalues, even modes first
+};
+struct DirectShape {
+    int n0 = 0, n1 = 0, n2 = 0;
+    DirectAxis ax[3];
 };
 
 // A Yee array of the EM mode: boost::multi_array with index bases, C order,
@@ -262,6 +295,8 @@ struct Ctx {
     bool pdl = true;                 // solver kernels launched with programmatic dependent launch
     int64_t solve_pre_launches = 0, solve_post_launches = 0;
     int64_t cycle_launches = 0;      // kernels in that graph
+    bool direct = false;             // corrections by fast diagonalisation instead of V-cycles
+    DirectShape dir;
     int mg_cta_start = -1;           // first level whose V-cycle runs inside one CTA
     double* red_partials = nullptr;  // block partial sums
     int red_blocks = 0;

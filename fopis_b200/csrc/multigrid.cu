@@ -15,9 +15,7 @@
 // faces are held during the solve and set afterwards by Field::
 // setBoundaryConditionPhi, src/Grid/Field.cpp:10-96). With every axis
 // periodic the mean of f is removed and phi is kept at zero mean.
-#include "internal.cuh"
-
-#include <utility>
+#include "direct.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -54,22 +52,6 @@ Lv lv(const MGLevel& m) {
 // kernel entry (griddepcontrol.launch_dependents) made them 2.61 ms.
 __device__ __forceinline__ void pdl_entry() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
-template <typename... KArgs, typename... Args>
-void launch_k(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-              Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    FOPIS_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
 }
 
 constexpr int kRowThreads = 128;
@@ -1075,6 +1057,16 @@ __global__ void reduce_partials_kernel(const double* partial, int n, int stride,
     if (threadIdx.x == 0) *out = v;
 }
 
+// Mean from per-block sums of f (every second partial).
+__global__ void mean_kernel(const double* partial, int n, double M, double* out) {
+    pdl_entry();
+    __shared__ double red[32];
+    double v = 0.0;
+    for (int t = threadIdx.x; t < n; t += blockDim.x) v += partial[2 * t];
+    v = bsum(v, red);
+    if (threadIdx.x == 0) *out = v / M;
+}
+
 // Threads of the row-walking FP64 kernels: one row of the contiguous axis per pass.
 int outer_threads(const Outer& O) { return std::min(kT, std::max(32, ((O.n2 + 31) / 32) * 32)); }
 
@@ -1405,6 +1397,15 @@ void mg_setup(Ctx& c) {
         n.scale = f.scale * 0.25;
         c.mg.push_back(n);
     }
+    c.direct = direct_fits(c.mg[0].n);
+    if (c.direct) {
+        MGLevel& l = c.mg[0];
+        FOPIS_CUDA(cudaMalloc(&l.f, sizeof(float) * l.size()));
+        direct_setup(c.dir, l.n, l.per);
+        c.red_blocks = std::max(kRedBlocks, direct_blocks(c.dir));
+        FOPIS_CUDA(cudaMalloc(&c.red_partials, sizeof(double) * 3 * c.red_blocks));
+        return;
+    }
     for (auto& l : c.mg) {
         FOPIS_CUDA(cudaMalloc(&l.u, sizeof(float) * l.size()));
         FOPIS_CUDA(cudaMalloc(&l.f, sizeof(float) * l.size()));
@@ -1450,7 +1451,44 @@ void mg_free(Ctx& c) {
     c.solve_state = 0;
     for (auto& l : c.mg) { cudaFree(l.u); cudaFree(l.f); cudaFree(l.r); }
     c.mg.clear();
+    direct_free(c.dir);
     if (c.red_partials) { cudaFree(c.red_partials); c.red_partials = nullptr; }
+}
+
+// The FP64 side of the direct correction's kernels.
+static DirectOuter direct_outer(const Ctx& c) {
+    const Outer O = make_outer(c);
+    DirectOuter d{};
+    d.cx = O.cx; d.cy = O.cy; d.cz = O.cz;
+    const int o[3] = {O.o0, O.o1, O.o2}, per[3] = {O.p0, O.p1, O.p2}, nref[3] = {O.nref0, O.nref1, O.nref2};
+    for (int a = 0; a < 3; ++a) { d.o[a] = o[a]; d.per[a] = per[a]; d.nref[a] = nref[a]; }
+    d.allper = O.p0 && O.p1 && O.p2;
+    d.eps0 = c.p.eps0;
+    d.inv_eps0 = O.inv_eps0;
+    return d;
+}
+
+// The first residual of a direct solve (with the mean of f before it when every
+// axis is periodic).
+static void direct_begin(Ctx& c, const Outer& O, const DirectStep& step) {
+    const DirectOuter D = direct_outer(c);
+    if (D.allper) {
+        c.launches += 2;
+        launch_k(c.pdl, fstats_kernel, kRedBlocks, outer_threads(O), 0, c.st, O, c.rho0, c.red_partials);
+        launch_k(c.pdl, mean_kernel, 1, 1024, 0, c.st, (const double*)c.red_partials, kRedBlocks,
+                 (double)O.n0 * O.n1 * O.n2, &c.d_sc->red[4]);
+    }
+    c.launches += direct_residual(c.dir, D, c.rho0, c.phi, c.mg[0].f, c.red_partials, step, c.pdl, c.st);
+    FOPIS_LAUNCH_CHECK();
+}
+
+// One refinement iteration of a direct solve: the correction and the residual
+// after it.
+static void direct_iteration(Ctx& c, const DirectStep& step) {
+    const DirectOuter D = direct_outer(c);
+    c.launches += direct_correct(c.dir, D, c.mg[0].f, c.phi, c.pdl, c.st);
+    c.launches += direct_residual(c.dir, D, c.rho0, c.phi, c.mg[0].f, c.red_partials, step, c.pdl, c.st);
+    FOPIS_LAUNCH_CHECK();
 }
 
 // Records one refinement iteration — V-cycle, FP64 correction, FP64 residual
@@ -1462,17 +1500,21 @@ static void ensure_cycle_graph(Ctx& c) {
     const int64_t before = c.launches;
     FOPIS_CUDA(cudaStreamBeginCapture(c.st, cudaStreamCaptureModeThreadLocal));
     try {
-        vcycle(c, 0);
-        if (!folds_correction(c)) {
+        if (c.direct) {
+            direct_iteration(c, DirectStep{c.d_sc, c.h_sc, 0, 0});
+        } else {
+            vcycle(c, 0);
+            if (!folds_correction(c)) {
+                ++c.launches;
+                launch_k(c.pdl, correct_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.phi, c.mg[0].u);
+            }
             ++c.launches;
-            launch_k(c.pdl, correct_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.phi, c.mg[0].u);
+            launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
+            ++c.launches;
+            launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 1, 0, &c.d_sc->red[2]);
+            FOPIS_LAUNCH_CHECK();
+            FOPIS_CUDA(cudaMemcpyAsync(&c.h_sc->red[2], &c.d_sc->red[2], sizeof(double), cudaMemcpyDeviceToHost, c.st));
         }
-        ++c.launches;
-        launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
-        ++c.launches;
-        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 1, 0, &c.d_sc->red[2]);
-        FOPIS_LAUNCH_CHECK();
-        FOPIS_CUDA(cudaMemcpyAsync(&c.h_sc->red[2], &c.d_sc->red[2], sizeof(double), cudaMemcpyDeviceToHost, c.st));
     } catch (...) {
         cudaGraph_t g = nullptr;
         cudaStreamEndCapture(c.st, &g);
@@ -1542,21 +1584,6 @@ void build_solve_graph(Ctx& c) {
     try {
         FOPIS_CUDA(cudaStreamBeginCapture(main_st, cudaStreamCaptureModeThreadLocal));
         capturing = true;
-        FOPIS_CUDA(cudaMemcpyAsync(&c.d_sc->red[6], &c.h_sc->red[6], 2 * sizeof(double), cudaMemcpyHostToDevice,
-                                   main_st));
-        ++c.launches;
-        launch_k(c.pdl, fstats_kernel, kRedBlocks, outer_threads(O), 0, main_st, O, c.rho0, c.red_partials);
-        ++c.launches;
-        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, main_st, c.red_partials, kRedBlocks, 2, 0, &c.d_sc->red[0]);
-        ++c.launches;
-        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, main_st, c.red_partials, kRedBlocks, 2, 1, &c.d_sc->red[1]);
-        ++c.launches;
-        launch_k(c.pdl, solve_prep_kernel, 1, 1, 0, main_st, c.d_sc, (double)M, allper ? 1 : 0);
-        ++c.launches;
-        launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, main_st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
-        ++c.launches;
-        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, main_st, c.red_partials, kRedBlocks, 1, 0, &c.d_sc->red[2]);
-        FOPIS_LAUNCH_CHECK();
         cudaStreamCaptureStatus status;
         cudaGraph_t graph = nullptr;
         const cudaGraphNode_t* deps = nullptr;
@@ -1564,9 +1591,27 @@ void build_solve_graph(Ctx& c) {
         FOPIS_CUDA(cudaStreamGetCaptureInfo(main_st, &status, nullptr, &graph, &deps, &ndeps));
         cudaGraphConditionalHandle handle;
         FOPIS_CUDA(cudaGraphConditionalHandleCreate(&handle, graph, 0, 0));
-        ++c.launches;
-        launch_k(c.pdl, solve_init_kernel, 1, 1, 0, main_st, c.d_sc, handle);
-        FOPIS_LAUNCH_CHECK();
+        if (c.direct) {
+            direct_begin(c, O, DirectStep{c.d_sc, c.h_sc, DIRECT_START | DIRECT_LOOP, handle});
+        } else {
+            FOPIS_CUDA(cudaMemcpyAsync(&c.d_sc->red[6], &c.h_sc->red[6], 2 * sizeof(double), cudaMemcpyHostToDevice,
+                                       main_st));
+            ++c.launches;
+            launch_k(c.pdl, fstats_kernel, kRedBlocks, outer_threads(O), 0, main_st, O, c.rho0, c.red_partials);
+            ++c.launches;
+            launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, main_st, c.red_partials, kRedBlocks, 2, 0, &c.d_sc->red[0]);
+            ++c.launches;
+            launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, main_st, c.red_partials, kRedBlocks, 2, 1, &c.d_sc->red[1]);
+            ++c.launches;
+            launch_k(c.pdl, solve_prep_kernel, 1, 1, 0, main_st, c.d_sc, (double)M, allper ? 1 : 0);
+            ++c.launches;
+            launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, main_st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
+            ++c.launches;
+            launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, main_st, c.red_partials, kRedBlocks, 1, 0, &c.d_sc->red[2]);
+            ++c.launches;
+            launch_k(c.pdl, solve_init_kernel, 1, 1, 0, main_st, c.d_sc, handle);
+            FOPIS_LAUNCH_CHECK();
+        }
         FOPIS_CUDA(cudaStreamGetCaptureInfo(main_st, &status, nullptr, &graph, &deps, &ndeps));
         cudaGraphNodeParams cp = {};
         cp.type = cudaGraphNodeTypeConditional;
@@ -1583,17 +1628,21 @@ void build_solve_graph(Ctx& c) {
         body_capturing = true;
         c.st = c.body_st;
         const int64_t b0 = c.launches;
-        vcycle(c, 0);
-        if (!folds_correction(c)) {
+        if (c.direct) {
+            direct_iteration(c, DirectStep{c.d_sc, c.h_sc, DIRECT_LOOP, handle});
+        } else {
+            vcycle(c, 0);
+            if (!folds_correction(c)) {
+                ++c.launches;
+                launch_k(c.pdl, correct_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.phi, c.mg[0].u);
+            }
             ++c.launches;
-            launch_k(c.pdl, correct_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.phi, c.mg[0].u);
+            launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
+            ++c.launches;
+            launch_k(c.pdl, solve_decide_kernel, 1, 1024, 0, c.st, (const double*)c.red_partials, kRedBlocks, c.d_sc,
+                     handle);
+            FOPIS_LAUNCH_CHECK();
         }
-        ++c.launches;
-        launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
-        ++c.launches;
-        launch_k(c.pdl, solve_decide_kernel, 1, 1024, 0, c.st, (const double*)c.red_partials, kRedBlocks, c.d_sc,
-                 handle);
-        FOPIS_LAUNCH_CHECK();
         body = c.launches - b0;
         c.st = main_st;
         cudaGraph_t body_graph = nullptr;
@@ -1609,7 +1658,8 @@ void build_solve_graph(Ctx& c) {
             launch_k(c.pdl, phi_shift_kernel, row_blocks((long long)O.n0 * O.n1), outer_threads(O), 0, main_st, O, c.phi, &c.d_sc->red[3]);
             FOPIS_LAUNCH_CHECK();
         }
-        FOPIS_CUDA(cudaMemcpyAsync(c.h_sc->red, c.d_sc->red, 16 * sizeof(double), cudaMemcpyDeviceToHost, main_st));
+        if (!c.direct)   // the direct residual writes the scalars to the pinned mirror itself
+            FOPIS_CUDA(cudaMemcpyAsync(c.h_sc->red, c.d_sc->red, 16 * sizeof(double), cudaMemcpyDeviceToHost, main_st));
         c.solve_post_launches = c.launches - p0;
         capturing = false;
         FOPIS_CUDA(cudaStreamEndCapture(main_st, &c.solve_graph));
@@ -1635,26 +1685,34 @@ void mg_solve_host_loop(Ctx& c, double tol, int max_cycles, double* res_out, dou
     Outer O = make_outer(c);
     const bool allper = O.p0 && O.p1 && O.p2;
     const long long M = (long long)O.n0 * O.n1 * O.n2;
-    ++c.launches;
-    launch_k(c.pdl, fstats_kernel, kRedBlocks, outer_threads(O), 0, c.st, O, c.rho0, c.red_partials);
-    ++c.launches;
-    launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 2, 0, &c.d_sc->red[0]);
-    ++c.launches;
-    launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 2, 1, &c.d_sc->red[1]);
-    FOPIS_LAUNCH_CHECK();
-    FOPIS_CUDA(cudaMemcpyAsync(c.h_sc->red, c.d_sc->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c.st));
-    FOPIS_CUDA(cudaStreamSynchronize(c.st));
-    const double fsum = c.h_sc->red[0], fsq = c.h_sc->red[1];
-    c.h_sc->red[4] = allper ? fsum / (double)M : 0.0;
-    FOPIS_CUDA(cudaMemcpyAsync(&c.d_sc->red[4], &c.h_sc->red[4], sizeof(double), cudaMemcpyHostToDevice, c.st));
-    double fnorm = std::sqrt(std::max(0.0, fsq - (allper ? fsum * fsum / (double)M : 0.0)));
-    if (!(fnorm > 0.0)) fnorm = 1.0;
-    ++c.launches;
-    launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
-    ++c.launches;
-    launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 1, 0, &c.d_sc->red[2]);
-    FOPIS_LAUNCH_CHECK();
-    double res = std::sqrt(read_red(c, 2));
+    double fnorm = 1.0, res = 0.0;
+    if (c.direct) {
+        direct_begin(c, O, DirectStep{c.d_sc, c.h_sc, DIRECT_START, 0});
+        FOPIS_CUDA(cudaStreamSynchronize(c.st));
+        fnorm = c.h_sc->red[5];
+        res = std::sqrt(c.h_sc->red[2]);
+    } else {
+        ++c.launches;
+        launch_k(c.pdl, fstats_kernel, kRedBlocks, outer_threads(O), 0, c.st, O, c.rho0, c.red_partials);
+        ++c.launches;
+        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 2, 0, &c.d_sc->red[0]);
+        ++c.launches;
+        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 2, 1, &c.d_sc->red[1]);
+        FOPIS_LAUNCH_CHECK();
+        FOPIS_CUDA(cudaMemcpyAsync(c.h_sc->red, c.d_sc->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+        FOPIS_CUDA(cudaStreamSynchronize(c.st));
+        const double fsum = c.h_sc->red[0], fsq = c.h_sc->red[1];
+        c.h_sc->red[4] = allper ? fsum / (double)M : 0.0;
+        FOPIS_CUDA(cudaMemcpyAsync(&c.d_sc->red[4], &c.h_sc->red[4], sizeof(double), cudaMemcpyHostToDevice, c.st));
+        fnorm = std::sqrt(std::max(0.0, fsq - (allper ? fsum * fsum / (double)M : 0.0)));
+        if (!(fnorm > 0.0)) fnorm = 1.0;
+        ++c.launches;
+        launch_k(c.pdl, outer_residual_march_kernel, kRedBlocks, kOuterThreads, 0, c.st, O, c.rho0, c.phi, c.mg[0].f, c.red_partials);
+        ++c.launches;
+        launch_k(c.pdl, reduce_partials_kernel, 1, 1024, 0, c.st, c.red_partials, kRedBlocks, 1, 0, &c.d_sc->red[2]);
+        FOPIS_LAUNCH_CHECK();
+        res = std::sqrt(read_red(c, 2));
+    }
     c.first_res = res / fnorm;
     int cycles = 0;
     while (res > tol * fnorm && cycles < max_cycles) {
@@ -1721,7 +1779,7 @@ int mg_solve(Ctx& c, double tol, int max_cycles) {
     } else {
         mg_solve_host_loop(c, tol, max_cycles, &res, &fnorm, &cycles);
     }
-    {   // the reference's pointwise measure on the state the solve reached (faces still held)
+    if (!c.direct) {   // the reference's pointwise measure on the state the solve reached (faces still held)
         const Outer O = make_outer(c);
         FOPIS_CUDA(cudaMemsetAsync(&c.d_sc->pointwise_bits, 0, sizeof(unsigned long long), c.st));
         ++c.launches;

@@ -1,0 +1,65 @@
+"""The fast-diagonalisation correction of the Poisson solve (direct.cu) at the
+sizes where its tiles, passes and folds end: single unknowns, odd and even
+periodic axes, axes around the multiples of the 8 modes, 16 matrix rows, 64
+lines and 128-mode passes it works in, and axes beyond its limit, which the
+multigrid cycle takes. The residual of the returned potential, formed here in
+FP64, has to meet the tolerance the solve reports; a correction lowers it by
+more than 1e-3, so two or three suffice for 1e-10 on any shape."""
+import numpy as np
+import pytest
+
+from fopis_b200 import RootGrid, _abi, config
+from fopis_b200.config import SpeciesInfo, make_params, plasma_units
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-10
+
+
+def residual(p, rho, phi):
+    """||f - A phi|| / ||f|| over the unknowns, faces held at zero, mean-free when every axis is periodic."""
+    dims = (p.nx, p.ny, p.nz)
+    per = [p.boundary[2 * a:2 * a + 1] == b"P" for a in range(3)]
+    inner = tuple(slice(1, n + 1) if q else slice(2, n) for n, q in zip(dims, per))
+    f = rho[inner] / p.eps0
+    if all(per):
+        f = f - f.mean()
+    u = phi[inner]
+    r = f - 6.0 * u
+    for a in range(3):
+        for d in (1, -1):
+            v = np.roll(u, d, axis=a)
+            if not per[a]:
+                np.moveaxis(v, a, 0)[0 if d == 1 else -1] = 0.0
+            r = r + v
+    return np.linalg.norm(r) / np.linalg.norm(f)
+
+
+@pytest.mark.parametrize("nxyz,boundary,direct", [
+    ((3, 3, 3), "DDDDDD", True), ((4, 3, 6), "DDNNDD", True), ((3, 4, 5), "PPPPPP", True),
+    ((17, 18, 19), "PPPPPP", True), ((33, 34, 35), "DDDDDD", True), ((66, 35, 34), "DDPPDD", True),
+    ((65, 130, 33), "PPDDPP", True), ((130, 131, 20), "DDPPNN", True), ((128, 72, 9), "PPPPPP", True),
+    ((145, 146, 60), "PPDDDD", True), ((261, 20, 12), "DDDDDD", True), ((20, 270, 16), "PPPPDD", True),
+    ((12, 10, 300), "NNDDPP", True), ((10, 9, 514), "DDDDDD", True), ((9, 8, 515), "DDDDDD", False)])
+def test_residual_meets_tolerance(gpu_available, nxyz, boundary, direct):
+    dx, dt = plasma_units()
+    sp = [SpeciesInfo("Electron", "ambient", 1.0, -1.0, 1e7, 1.0, 1)]
+    p, norm = make_params(nxyz, boundary, dx, dt, sp, tol=TOL, guess=_abi.GUESS_ZERO)
+    g = RootGrid(config.SimConfig(params=p, norm=norm, species=sp))
+    rng = np.random.default_rng(31)
+    shape = tuple(n + 2 for n in nxyz)
+    smooth = sum(np.cos(0.7 + 2.0 * np.pi * np.arange(s) / s).reshape([-1 if q == a else 1 for q in range(3)])
+                 for a, s in enumerate(shape))
+    rho = rng.standard_normal(shape) * 1e6 + 4e6 * smooth
+    g.set_field(_abi.FIELD_RHO0, rho)
+    rc = g.solvePoisson()
+    st = g.stats()
+    phi = g.getPhi()
+    g.close()
+    if direct:
+        assert rc == 0 and st.converged and 1 <= st.vcycles_last <= 3
+        # the reported residual is the last one formed; storing phi adds its rounding, 12 ulp of max |phi| a node
+        eps = 12 * 2.0 ** -52 * np.abs(phi).max() * np.sqrt(phi.size) / np.linalg.norm(rho / p.eps0)
+        assert residual(p, rho, phi) <= TOL + eps
+    else:
+        assert rc == 0 and st.vcycles_last > 3
