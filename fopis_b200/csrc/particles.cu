@@ -687,7 +687,7 @@ __device__ __forceinline__ void em_warp_move_current(const EdgeFix& J, bool had,
 // [a.lo, count): the old-cell half of the current, the move with the boundary
 // rules, the new-cell half, the body test and the rho deposit
 // (updateParticlePositionEM, then updateRho's per-particle part,
-// RootGridField.cpp:1168-1196). push_brick_kernel<.., true> takes the sorted bricks.
+// RootGridField.cpp:1168-1196). em_brick_kernel takes the sorted bricks.
 __global__ void __launch_bounds__(kThreads) em_tail_kernel(PushArgs a, EdgeFix J) {
     const long long n = (long long)min(*a.count, (unsigned long long)a.cap);
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -860,13 +860,55 @@ __device__ __forceinline__ void corners_from_moments(unsigned long long M[8]) {
             if (!(T & axis)) M[T] = (M[T] << kDepositBits) - M[T | axis];
 }
 
-template <int MINB, bool EM>
-__global__ void __launch_bounds__(kBrickThreads, MINB) push_brick_kernel(PushArgs a, const int32_t* brick_start,
-                                                                         EdgeFix J) {
+// End of a segment: the occupied cells' moments become corner weights, summed
+// per node in the tile (low plane, high plane) and added to the species'
+// accumulator. Returns true when a node sum wrapped past 2^64.
+template <int THREADS>
+__device__ __forceinline__ bool flush_moments(const unsigned* mom, unsigned* t_lo, const PushArgs& a, int wx0, int wy0,
+                                              int wz0) {
+    unsigned* const t_hi = t_lo + kWinNodes;
+    bool wrap = false;
+    for (int t = threadIdx.x; t < 2 * kWinNodes; t += THREADS) t_lo[t] = 0u;
+    __syncthreads();
+    for (int t = threadIdx.x; t < kWinCells; t += THREADS) {
+        const unsigned n = mom[t];
+        if (!n) continue;
+        const unsigned* m = mom + t;
+        unsigned long long M[8];
+        M[0] = n;                                                      // {}
+        M[4] = m[1 * kWinCells];                                       // {x}: A
+        M[2] = m[2 * kWinCells];                                       // {y}: B
+        M[1] = m[3 * kWinCells];                                       // {z}: D
+        M[6] = m[4 * kWinCells] + ((unsigned long long)m[5 * kWinCells] << 17);    // {x,y}: AB
+        M[5] = m[6 * kWinCells] + ((unsigned long long)m[7 * kWinCells] << 17);    // {x,z}: AD
+        M[3] = m[8 * kWinCells] + ((unsigned long long)m[9 * kWinCells] << 17);    // {y,z}: BD
+        M[7] = m[10 * kWinCells] + ((unsigned long long)m[11 * kWinCells] << 17) +
+               ((unsigned long long)m[12 * kWinCells] << 34);                      // {x,y,z}: ABD
+        corners_from_moments(M);
+        const int x = t / (kCY * kCZ), y = (t / kCZ) % kCY, z = t % kCZ;
+        const int nb = (x * kNY + y) * kNZ + z;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const int off = ((c >> 2) ? kNY * kNZ : 0) + (((c >> 1) & 1) ? kNZ : 0) + (c & 1);
+            wrap |= tile_add_checked(t_lo, t_hi, nb + off, M[c]);
+        }
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < kWinNodes; t += THREADS) {
+        const unsigned long long v = (unsigned long long)t_lo[t] | ((unsigned long long)t_hi[t] << 32);
+        if (!v) continue;
+        const int x = wx0 + t / (kNY * kNZ), y = wy0 + (t / kNZ) % kNY, z = wz0 + t % kNZ;
+        const unsigned long long old = atomicAdd(a.rho + lin(a.g, x, y, z), v);
+        wrap |= old + v < old;
+    }
+    __syncthreads();
+    return wrap;
+}
+
+__global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a, const int32_t* brick_start) {
     __shared__ __align__(16) unsigned s_mom[kPlanes * kWinCells];
     __shared__ __align__(16) unsigned long long s_batch[kBatchPad];    // batch entries; node tile in the epilogue
     unsigned* const t_lo = reinterpret_cast<unsigned*>(s_batch);
-    unsigned* const t_hi = t_lo + kWinNodes;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b = blockIdx.x;
     const int bi = b / (a.g.nb[1] * a.g.nb[2]), bj = (b / a.g.nb[2]) % a.g.nb[1], bk = b % a.g.nb[2];
@@ -910,21 +952,7 @@ __global__ void __launch_bounds__(kBrickThreads, MINB) push_brick_kernel(PushArg
                     const long long idx = c0 + q;
                     bool live = cell[r] >= 0;
                     PState st{0, 0, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                    if constexpr (EM) {
-                        // the EM step: velocities were updated by em_velocity_kernel; the move
-                        // carries the two halves of the charge-conserving current
-                        const bool had = live;
-                        if (live) {
-                            unpack_cell(cell[r], st.i, st.j, st.k);
-                            st.ox = f[r][0]; st.oy = f[r][1]; st.oz = f[r][2];
-                            st.vx = f[r][3]; st.vy = f[r][4]; st.vz = f[r][5];
-                            if (J.B) em_kick(a, J.B, st);
-                        }
-                        const int oi = st.i, oj = st.j, ok = st.k;
-                        const float o0[3] = {st.ox, st.oy, st.oz};
-                        if (live) live = move_boundary(a, st);
-                        em_warp_move_current(J, had, oi, oj, ok, o0, st, live);
-                    } else if (live) {
+                    if (live) {
                         unpack_cell(cell[r], st.i, st.j, st.k);
                         st.ox = f[r][0]; st.oy = f[r][1]; st.oz = f[r][2];
                         st.vx = f[r][3]; st.vy = f[r][4]; st.vz = f[r][5];
@@ -979,46 +1007,273 @@ __global__ void __launch_bounds__(kBrickThreads, MINB) push_brick_kernel(PushArg
             }
             __syncthreads();
         }
-        // occupied cells: moments -> corner weights -> node tile (in the batch buffer)
-        for (int t = tid; t < 2 * kWinNodes; t += kBrickThreads) t_lo[t] = 0u;
-        __syncthreads();
-        for (int t = tid; t < kWinCells; t += kBrickThreads) {
-            const unsigned n = s_mom[t];
-            if (!n) continue;
-            const unsigned* m = s_mom + t;
-            unsigned long long M[8];
-            M[0] = n;                                                      // {}
-            M[4] = m[1 * kWinCells];                                       // {x}: A
-            M[2] = m[2 * kWinCells];                                       // {y}: B
-            M[1] = m[3 * kWinCells];                                       // {z}: D
-            M[6] = m[4 * kWinCells] + ((unsigned long long)m[5 * kWinCells] << 17);    // {x,y}: AB
-            M[5] = m[6 * kWinCells] + ((unsigned long long)m[7 * kWinCells] << 17);    // {x,z}: AD
-            M[3] = m[8 * kWinCells] + ((unsigned long long)m[9 * kWinCells] << 17);    // {y,z}: BD
-            M[7] = m[10 * kWinCells] + ((unsigned long long)m[11 * kWinCells] << 17) +
-                   ((unsigned long long)m[12 * kWinCells] << 34);                      // {x,y,z}: ABD
-            corners_from_moments(M);
-            const int x = t / (kCY * kCZ), y = (t / kCZ) % kCY, z = t % kCZ;
-            const int nb = (x * kNY + y) * kNZ + z;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const int off = ((c >> 2) ? kNY * kNZ : 0) + (((c >> 1) & 1) ? kNZ : 0) + (c & 1);
-                wrap |= tile_add_checked(t_lo, t_hi, nb + off, M[c]);
-            }
-        }
-        __syncthreads();
-        for (int t = tid; t < kWinNodes; t += kBrickThreads) {
-            const unsigned long long v = (unsigned long long)t_lo[t] | ((unsigned long long)t_hi[t] << 32);
-            if (!v) continue;
-            const int x = wx0 + t / (kNY * kNZ), y = wy0 + (t / kNZ) % kNY, z = wz0 + t % kNZ;
-            const unsigned long long old = atomicAdd(a.rho + lin(a.g, x, y, z), v);
-            wrap |= old + v < old;
-        }
-        __syncthreads();
+        wrap |= flush_moments<kBrickThreads>(s_mom, t_lo, a, wx0, wy0, wz0);
     }
     if (wrap) atomicOr(&a.sc->status, (unsigned)FOPIS_DEV_RHO_OVERFLOW);
     const double tot = block_sum(e2);
     if (tid == 0 && tot != 0.0) atomicAdd(&a.sc->energy[a.s], tot);
     const double np = block_sum(npushed), nk = block_sum(nkept);
+    if (tid == 0) {
+        if (np > 0.0) atomicAdd(&a.sc->pushed[a.s], (unsigned long long)np);
+        if (nk > 0.0) atomicAdd(&a.sc->survived[a.s], (unsigned long long)nk);
+    }
+}
+
+// ------------------------------------------------------------------ EM brick push
+// em_brick_kernel: the EM step's particle pass over the brick-sorted particles
+// (velocity when J.B is set, move with the boundary rules, zigzag current, body
+// test, rho deposit), one brick per CTA.
+//
+// The current goes to a tile of fixed-point edge sums over the window of the rho
+// moments, a low plane of 16-bit pieces and a high plane of the rest (32-bit
+// words, no-return shared atomics; a segment adds at most 2 x 7168 pieces to a
+// word, so neither plane wraps), added to the species' int64 sums once per
+// segment. Lanes that hold consecutive, same-cell particles would serialise on
+// the tile's words, so a batch keeps each particle's start offsets, velocity and
+// cells in shared memory and is read back with lanes 32 places apart, i.e. in
+// different cells: four groups of warps take the rho moments and the edges of
+// one direction each (summing runs of same-cell particles in registers first,
+// as the ES pass does, made the warp take the flush at nearly every entry once
+// particles have drifted: 7.0 ms). Moves that change
+// their cell (a tenth of the electrons) are listed and their two halves added
+// one by one; particles whose cells lie outside the window use global atomics.
+// Warp sums and 64-bit global atomics for every particle (em_warp_move_current)
+// took 11.0 ms at 128^3 (1.34e8 particles), this 7.0 (1.07 TB/s of the 56 B a
+// particle); it is bound by the shared-memory and gather wavefronts (69 % of
+// the LSU data path busy) and the latency of the gather. One low word with a
+// carry instead of two pieces: 7.3. 512 threads, because the tile and the batch
+// leave room for two CTAs per SM.
+constexpr int kEmThreads = 512;
+constexpr int kEmRun = 4 * kBatch / kEmThreads;          // entries per thread of a group
+constexpr int kEdge0 = kCX * kNY * kNZ, kEdge1 = kNX * kCY * kNZ, kEdge2 = kNX * kNY * kCZ;   // window edges along x, y, z
+constexpr int kEdges = kEdge0 + kEdge1 + kEdge2;
+struct EmTile {
+    unsigned mom[kPlanes * kWinCells];
+    unsigned long long batch[kBatchPad];                 // rho entries; node tile at the end of a segment
+    unsigned lo[kEdges], hi[kEdges];                     // edge sums
+    float o[3][kBatchPad], v[3][kBatchPad];              // start offsets and velocity
+    unsigned cells[kBatchPad];                           // start cell of a move that stays; else none, new and old cell, 10 bits each
+    unsigned short list[kBatch];                         // entries that change their cell
+    int listed[2];                                       // of this batch and the next
+};
+static_assert(kEmRun * kEmThreads == 4 * kBatch && 32 % kEmRun == 0, "a run lies in one lane's 32 entries");
+
+// A window cell as x, y, z in 3 + 3 + 4 bits, three of which fit a word; kNoCell is none.
+constexpr unsigned kNoCell = 0x3FFu;
+static_assert(kCX <= 8 && kCY <= 8 && kCZ <= 15, "window cell code");
+__device__ __forceinline__ unsigned cell_code(int x, int y, int z) { return (unsigned)(x << 7 | y << 4 | z); }
+
+// Word of edge term q (em_terms order: +1 along the first, then the second other
+// axis) of direction d at a window cell.
+__device__ __forceinline__ int edge_word(int d, unsigned code) {
+    const int x = (int)(code >> 7), y = (int)(code >> 4) & 7, z = (int)code & 15;
+    return d == 0 ? (x * kNY + y) * kNZ + z
+                  : d == 1 ? kEdge0 + (x * kCY + y) * kNZ + z : kEdge0 + kEdge1 + (x * kNY + y) * kCZ + z;
+}
+__device__ __forceinline__ int edge_step(int d, int q) {
+    const int first = d == 0 ? kNZ : (d == 1 ? kCY * kNZ : kNY * kCZ), second = d == 2 ? kCZ : 1;
+    return ((q & 1) ? first : 0) + ((q >> 1) ? second : 0);
+}
+__device__ __forceinline__ void edge_add(EmTile& T, int d, unsigned code, const int t[4]) {
+    const int w = edge_word(d, code);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        atomicAdd(T.lo + w + edge_step(d, q), (unsigned)t[q] & 0xFFFFu);
+        atomicAdd(T.hi + w + edge_step(d, q), (unsigned)(t[q] >> 16));
+    }
+}
+// The four edge terms of one direction of em_terms / em_terms_same: flux and the
+// weights of the other two axes, cross = the product term of a whole move.
+__device__ __forceinline__ void edge_terms(float flux, float wb, float wc, float cross, int t[4]) {
+    const float s = kCurrentScale * flux;
+    t[0] = __float2int_rn(s * ((1.0f - wb) * (1.0f - wc) + cross));
+    t[1] = __float2int_rn(s * (wb * (1.0f - wc) - cross));
+    t[2] = __float2int_rn(s * ((1.0f - wb) * wc - cross));
+    t[3] = __float2int_rn(s * (wb * wc + cross));
+}
+
+// The two halves of a cell-changing move on the edges of direction d.
+__device__ __forceinline__ void edge_cross(EmTile& T, int entry, int d) {
+    const unsigned cells = T.cells[entry];
+    PState st{0, 0, 0, T.o[0][entry], T.o[1][entry], T.o[2][entry], T.v[0][entry], T.v[1][entry], T.v[2][entry]};
+    float f[3], w[3];
+    int t[4];
+    em_half_old(st, f, w);
+    const int b = d == 0 ? 1 : 0, c = d == 2 ? 1 : 2;
+    edge_terms(f[d], w[b], w[c], 0.0f, t);
+    edge_add(T, d, cells >> 20, t);
+    const unsigned fresh = (cells >> 10) & kNoCell;
+    if (fresh == kNoCell) return;
+    st.ox += st.vx; st.oy += st.vy; st.oz += st.vz;
+    st.ox -= floorf(st.ox); st.oy -= floorf(st.oy); st.oz -= floorf(st.oz);
+    em_half_new(st, f, w);
+    edge_terms(f[d], w[b], w[c], 0.0f, t);
+    edge_add(T, d, fresh, t);
+}
+
+// A particle's current with global atomics, both halves.
+__device__ __noinline__ void em_lane_current(const EdgeFix& J, int oi, int oj, int ok, float ox, float oy, float oz,
+                                             const PState& st, bool live) {
+    const float v[3] = {st.vx, st.vy, st.vz}, o0[3] = {ox, oy, oz};
+    int t[12];
+    if (live && st.i == oi && st.j == oj && st.k == ok) {
+        em_terms_same(o0, v, t);
+        live = false;
+    } else {
+        PState s0 = st;
+        s0.ox = ox; s0.oy = oy; s0.oz = oz;
+        float f[3], w[3];
+        em_half_old(s0, f, w);
+        em_terms(f, w, t);
+    }
+    for (int q = 0; q < 12; ++q)
+        if (t[q]) atomicAdd(em_term_ptr(J, oi, oj, ok, q), (unsigned long long)(long long)t[q]);
+    if (!live) return;
+    float f[3], w[3];
+    em_half_new(st, f, w);
+    em_terms(f, w, t);
+    for (int q = 0; q < 12; ++q)
+        if (t[q]) atomicAdd(em_term_ptr(J, st.i, st.j, st.k, q), (unsigned long long)(long long)t[q]);
+}
+
+__global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, const int32_t* brick_start, EdgeFix J) {
+    extern __shared__ __align__(16) unsigned char em_smem[];
+    EmTile& T = *reinterpret_cast<EmTile*>(em_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.x;
+    const int bi = b / (a.g.nb[1] * a.g.nb[2]), bj = (b / a.g.nb[2]) % a.g.nb[1], bk = b % a.g.nb[2];
+    const int wx0 = bi * kBX - kHalo, wy0 = bj * kBY - kHalo, wz0 = bk * kBZ - kHalo;
+    const long long p0 = brick_start[b], p1 = brick_start[b + 1];
+    if (p0 == p1) return;
+    int body = 0;
+    for (int t = tid; t < kWinCells; t += kEmThreads) {
+        const int x = wx0 + t / (kCY * kCZ), y = wy0 + (t / kCZ) % kCY, z = wz0 + t % kCZ;
+        if (a.cellmap && x >= 0 && y >= 0 && z >= 0 && x < a.g.cx - 1 && y < a.g.cy - 1 && z < a.g.cz - 1 &&
+            a.cellmap[lin(a.g, x, y, z)] != 0)
+            body = 1;
+    }
+    const bool window_body = __syncthreads_or(body) != 0;
+    int npushed = 0, nkept = 0;
+    bool wrap = false;
+    for (long long s0 = p0; s0 < p1; s0 += kSegment) {
+        const long long s1 = min(p1, s0 + (long long)kSegment);
+        for (int t = tid; t < kPlanes * kWinCells; t += kEmThreads) T.mom[t] = 0u;
+        for (int t = tid; t < kEdges; t += kEmThreads) { T.lo[t] = 0u; T.hi[t] = 0u; }
+        if (tid < 2) T.listed[tid] = 0;
+        int turn = 0;
+        __syncthreads();
+        for (long long c0 = s0; c0 < s1; c0 += kBatch, turn ^= 1) {
+#pragma unroll 1
+            for (int h = 0; h < kBatch / kEmThreads; ++h) {
+                const int q = h * kEmThreads + tid;
+                const long long idx = c0 + q;
+                const int32_t cell = idx < s1 ? a.p.cell[idx] : -1;
+                const bool had = cell >= 0;
+                bool live = had;
+                PState st{0, 0, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                float ox = 0.f, oy = 0.f, oz = 0.f;
+                int oi = 0, oj = 0, ok = 0;
+                if (live) {
+                    unpack_cell(cell, oi, oj, ok);
+                    st.i = oi; st.j = oj; st.k = ok;
+                    ox = a.p.ox[idx]; oy = a.p.oy[idx]; oz = a.p.oz[idx];
+                    st.ox = ox; st.oy = oy; st.oz = oz;
+                    st.vx = a.p.vx[idx]; st.vy = a.p.vy[idx]; st.vz = a.p.vz[idx];
+                    if (J.B) em_kick(a, J.B, st);
+                    live = move_boundary(a, st);
+                }
+                const int li = st.i - wx0, lj = st.j - wy0, lk = st.k - wz0;
+                const bool inwin = (unsigned)li < (unsigned)kCX && (unsigned)lj < (unsigned)kCY && (unsigned)lk < (unsigned)kCZ;
+                const int wc = (li * kCY + lj) * kCZ + lk;
+                const int mi = oi - wx0, mj = oj - wy0, mk = ok - wz0;
+                const bool oldin = (unsigned)mi < (unsigned)kCX && (unsigned)mj < (unsigned)kCY && (unsigned)mk < (unsigned)kCZ;
+                const unsigned was = cell_code(mi, mj, mk), now = live ? cell_code(li, lj, lk) : kNoCell;
+                const int e = bpad(q);
+                // the current: tile entry, listed move, or global atomics
+                const bool tiled = had && oldin && (inwin || !live);
+                const bool crosses = tiled && was != now;
+                if (had && !tiled) em_lane_current(J, oi, oj, ok, ox, oy, oz, st, live);
+                T.cells[e] = !tiled ? kNoCell : (crosses ? kNoCell | now << 10 | was << 20 : was);
+                T.o[0][e] = ox; T.o[1][e] = oy; T.o[2][e] = oz;
+                T.v[0][e] = st.vx; T.v[1][e] = st.vy; T.v[2][e] = st.vz;
+                const unsigned m = __ballot_sync(kFull, crosses);
+                if (m) {
+                    int at = 0;
+                    if (lane == __ffs(m) - 1) at = atomicAdd(&T.listed[turn], __popc(m));
+                    at = __shfl_sync(kFull, at, __ffs(m) - 1);
+                    if (crosses) T.list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)e;
+                }
+                const bool test = live && (window_body || !inwin);
+                if (__any_sync(kFull, test) && absorb_check(a, st, test)) live = false;
+                const unsigned qa = (unsigned)__float2int_rn(st.ox * kDepositScale);
+                const unsigned qb = (unsigned)__float2int_rn(st.oy * kDepositScale);
+                const unsigned qd = (unsigned)__float2int_rn(st.oz * kDepositScale);
+                T.batch[e] = (live && inwin) ? ((unsigned long long)wc | ((unsigned long long)qa << 10) |
+                                                ((unsigned long long)qb << 28) | ((unsigned long long)qd << 46))
+                                             : kNoDeposit;
+                if (live && !inwin) wrap |= global_deposit(a.rho, a.g, lin(a.g, st.i, st.j, st.k), qa, qb, qd);
+                npushed += had;
+                nkept += live;
+                if (had) {
+                    a.p.cell[idx] = live ? pack_cell(st.i, st.j, st.k) : -1;
+                    a.p.ox[idx] = st.ox; a.p.oy[idx] = st.oy; a.p.oz[idx] = st.oz;
+                    if (J.B) { a.p.vx[idx] = st.vx; a.p.vy[idx] = st.vy; a.p.vz[idx] = st.vz; }
+                }
+            }
+            __syncthreads();
+            const int group = warp / (kEmThreads / 128);
+            // entries lane * 32 + ... of the batch, padded: lanes are 33 words apart
+            const int first = lane * (kBatch / 32 + 1) + (warp % (kEmThreads / 128)) * kEmRun;
+            if (group == 3) {
+#pragma unroll 2
+                for (int r = 0; r < kEmRun; ++r) {
+                    const unsigned long long en = T.batch[first + r];
+                    const int wc = (int)(en & 0x3FFull);
+                    if (wc == (int)kNoDeposit) continue;
+                    MomentSum one;
+                    one.add((unsigned)(en >> 10) & 0x3FFFFu, (unsigned)(en >> 28) & 0x3FFFFu, (unsigned)(en >> 46));
+                    one.flush(T.mom, wc);
+                }
+            } else {
+                const int ob = group == 0 ? 1 : 0, oc = group == 2 ? 1 : 2;
+                const float *va = T.v[group], *vb = T.v[ob], *vc = T.v[oc], *xb = T.o[ob], *xc = T.o[oc];
+#pragma unroll 2
+                for (int r = 0; r < kEmRun; ++r) {
+                    const int e = first + r;
+                    const unsigned code = T.cells[e] & kNoCell;
+                    if (code == kNoCell) continue;
+                    const float b1 = vb[e], c1 = vc[e];
+                    int t[4];
+                    edge_terms(va[e], xb[e] + 0.5f * b1, xc[e] + 0.5f * c1, (0.25f * b1) * (0.25f * c1), t);
+                    edge_add(T, group, code, t);
+                }
+            }
+            if (tid == 0) T.listed[turn ^ 1] = 0;
+            const int listed = T.listed[turn];
+            for (int t = tid; t < 3 * listed; t += kEmThreads) edge_cross(T, T.list[t / 3], t % 3);
+            __syncthreads();
+        }
+        wrap |= flush_moments<kEmThreads>(T.mom, reinterpret_cast<unsigned*>(T.batch), a, wx0, wy0, wz0);
+        for (int t = tid; t < kEdges; t += kEmThreads) {
+            const long long v = (long long)T.lo[t] + ((long long)(int)T.hi[t] << 16);
+            if (v == 0) continue;
+            unsigned long long* out;
+            if (t < kEdge0) {
+                const int x = wx0 + t / (kNY * kNZ), y = wy0 + (t / kNZ) % kNY, z = wz0 + t % kNZ;
+                out = J.x + ((long long)x * J.cy + y) * J.cz + z;
+            } else if (t < kEdge0 + kEdge1) {
+                const int u = t - kEdge0, x = wx0 + u / (kCY * kNZ), y = wy0 + (u / kNZ) % kCY, z = wz0 + u % kNZ;
+                out = J.y + ((long long)x * (J.cy - 1) + y) * J.cz + z;
+            } else {
+                const int u = t - kEdge0 - kEdge1, x = wx0 + u / (kNY * kCZ), y = wy0 + (u / kCZ) % kNY, z = wz0 + u % kCZ;
+                out = J.z + ((long long)x * J.cy + y) * (J.cz - 1) + z;
+            }
+            atomicAdd(out, (unsigned long long)v);
+        }
+        __syncthreads();
+    }
+    if (wrap) atomicOr(&a.sc->status, (unsigned)FOPIS_DEV_RHO_OVERFLOW);
+    const double np = block_sum((double)npushed), nk = block_sum((double)nkept);
     if (tid == 0) {
         if (np > 0.0) atomicAdd(&a.sc->pushed[a.s], (unsigned long long)np);
         if (nk > 0.0) atomicAdd(&a.sc->survived[a.s], (unsigned long long)nk);
@@ -2339,7 +2594,7 @@ void launch_push(Ctx& c, bool vel, bool pos, bool dep) {
         } else if (vel && pos && dep && c.sorted_n[s] > 0 && c.brick_start[s]) {
             PushArgs a = push_args<float>(c, s);
             ++c.launches;
-            push_brick_kernel<4, false><<<brick_count(c), kBrickThreads, 0, c.st>>>(a, c.brick_start[s], EdgeFix{});
+            push_brick_kernel<<<brick_count(c), kBrickThreads, 0, c.st>>>(a, c.brick_start[s]);
             a.lo = c.sorted_n[s];
             ++c.launches;
             push_kernel<float, true, true, true><<<grid_for(std::max<int64_t>(c.cap[s] - a.lo, 1)), kThreads, 0, c.st>>>(a);
@@ -2365,7 +2620,7 @@ void launch_em_velocity(Ctx& c) {
 }
 
 // The mixed mode's EM particle pass: per species the brick-sorted slots with
-// push_brick_kernel<.., true> and the appended tail with em_tail_kernel (move,
+// em_brick_kernel and the appended tail with em_tail_kernel (move,
 // fixed-point current halves, body test, rho deposit), then J in FP64 and its
 // periodic folds. With kick the same pass gives the velocity update first
 // (the caller's choice when no particle is emitted between the two updates).
@@ -2382,7 +2637,8 @@ void launch_em_move(Ctx& c, bool kick) {
         PushArgs a = push_args<float>(c, s);
         if (c.sorted_n[s] > 0 && c.brick_start[s]) {
             ++c.launches;
-            push_brick_kernel<3, true><<<brick_count(c), kBrickThreads, 0, c.st>>>(a, c.brick_start[s], J);
+            FOPIS_CUDA(cudaFuncSetAttribute(em_brick_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EmTile)));
+            em_brick_kernel<<<brick_count(c), kEmThreads, sizeof(EmTile), c.st>>>(a, c.brick_start[s], J);
             a.lo = c.sorted_n[s];
         }
         ++c.launches;
