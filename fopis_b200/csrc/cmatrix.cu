@@ -2,8 +2,10 @@
 // per-step equipotential correction.
 //
 // Capacity matrix (RootGrid::initializeObjectsCmatrix, RootGridObject.cpp:77-148):
-// column c of B holds phi at every surface node for rho = 1 at surface node c
-// (one multigrid solve per column); C = B^-1 by in-place Gauss-Jordan
+// column c of B holds phi at every surface node for rho = 1 at surface node c:
+// values of the grid's Green's function, from one table over node differences
+// and sums (one multigrid or direct solve per column where a surface node is
+// not an unknown of the solve); C = B^-1 by blocked in-place Gauss-Jordan
 // elimination in FP64 on the device (B is symmetric positive definite, so no
 // pivoting). Per step (Spacecraft::redistributeChargeForPerfectConductor,
 // Spacecraft.cpp:708-758): V = (sum_ij C_ij phi_j + Q) / sum_ij C_ij, or the
@@ -45,28 +47,180 @@ __global__ void gather_kernel(const double* phi, const int32_t* nodes, int n, do
 
 __global__ void set_node_kernel(double* a, long long idx, double v) { a[idx] = v; }
 
-// Gauss-Jordan step k: copy row k and column k aside.
-__global__ void gj_copy_kernel(const double* A, int n, int k, double* rowk, double* colk) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        rowk[t] = A[(long long)k * n + t];
-        colk[t] = A[(long long)t * n + k];
+// Green's function of the 7-point operator with the solve's closure. Along an
+// axis between held faces the eigenvectors are sines, and a product of two is
+// half a difference of cosines of the node difference and the node sum; along a
+// periodic axis only the difference enters. So phi at node r for a charge at
+// node c is a signed sum of at most eight entries of
+//   T[u][v][w] = sum_klm Ca[k][u] Cb[l][v] Cc[m][w] / (lambda_k + lambda_l + lambda_m)
+// over the offsets u, v, w the surface has (differences, then sums), three small
+// FP64 contractions. The mean mode of an all-periodic box is left out, as the
+// solve leaves it out. 47^3 unknowns, 218 nodes: 190 ms of solves by V-cycles,
+struct GreenAxis {
+    int n, per;      // unknowns, periodic
+    int lo, span;    // smallest 1-based unknown of the surface, largest minus smallest
+    int count;       // offsets: span + 1 differences, then 2 span + 1 sums between held faces
+    double* cosines; // [n][count]
+    double* lambda;  // [n]
+};
+
+__global__ void green_axis_kernel(GreenAxis x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < x.n * x.count; t += gridDim.x * blockDim.x) {
+        const int k = t / x.count, u = t - k * x.count;
+        const int offset = u <= x.span ? u : 2 * x.lo + (u - x.span - 1);
+        if (x.per) {
+            x.cosines[t] = cospi(2.0 * (double)(((long long)offset * k) % x.n) / x.n) / x.n;
+            if (u == 0) { const double q = sinpi((double)k / x.n); x.lambda[k] = 4.0 * q * q; }
+        } else {
+            x.cosines[t] = cospi((double)(((long long)offset * (k + 1)) % (2 * (x.n + 1))) / (x.n + 1)) / (x.n + 1);
+            if (u == 0) { const double q = sinpi(0.5 * (k + 1) / (x.n + 1)); x.lambda[k] = 4.0 * q * q; }
+        }
     }
 }
-// In-place Gauss-Jordan inversion step k (no pivoting).
-__global__ void gj_update_kernel(double* A, int n, int k, const double* rowk, const double* colk, unsigned* bad) {
-    const double akk = colk[k];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !(akk > 0.0)) atomicOr(bad, 1u);
-    const double p = 1.0 / akk;
+
+// R[k][l][w] = sum_m Cc[m][w] / (lambda_k + lambda_l + lambda_m): kGreenL values
+// of l per CTA share the reads of Cc.
+constexpr int kGreenL = 4, kGreenThreads = 128;
+__global__ void __launch_bounds__(kGreenThreads) green_sum_kernel(GreenAxis a, GreenAxis b, GreenAxis c, double* R) {
+    extern __shared__ double inv[];   // [kGreenL][c.n]
+    const int k = blockIdx.y, l0 = blockIdx.x * kGreenL;
+    for (int t = threadIdx.x; t < kGreenL * c.n; t += kGreenThreads) {
+        const int l = min(l0 + t / c.n, b.n - 1);
+        const double e = a.lambda[k] + b.lambda[l] + c.lambda[t % c.n];
+        inv[t] = e > 0.0 ? 1.0 / e : 0.0;
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < c.count; w += kGreenThreads) {
+        double s[kGreenL] = {};
+#pragma unroll 4
+        for (int m = 0; m < c.n; ++m) {
+            const double q = c.cosines[(long long)m * c.count + w];
+#pragma unroll
+            for (int e = 0; e < kGreenL; ++e) s[e] += q * inv[e * c.n + m];
+        }
+        for (int e = 0; e < kGreenL && l0 + e < b.n; ++e) R[((long long)k * b.n + l0 + e) * c.count + w] = s[e];
+    }
+}
+
+// out[o][u][q] = sum_k C[k][u] in[o][k][q]: one axis' contraction, q of the
+// `inner` trailing values per thread, kGreenU offsets u of it.
+constexpr int kGreenU = 4;
+__global__ void __launch_bounds__(kGreenThreads) green_contract_kernel(GreenAxis x, const double* in, int inner,
+                                                                       double* out) {
+    const int q = blockIdx.x * kGreenThreads + threadIdx.x, u0 = blockIdx.y * kGreenU;
+    if (q >= inner) return;
+    in += (long long)blockIdx.z * x.n * inner + q;
+    double s[kGreenU] = {};
+#pragma unroll 4
+    for (int k = 0; k < x.n; ++k) {
+        const double v = in[(long long)k * inner];
+#pragma unroll
+        for (int e = 0; e < kGreenU; ++e) s[e] += x.cosines[(long long)k * x.count + min(u0 + e, x.count - 1)] * v;
+    }
+    for (int e = 0; e < kGreenU && u0 + e < x.count; ++e)
+        out[((long long)blockIdx.z * x.count + u0 + e) * inner + q] = s[e];
+}
+
+// B from the table; u: the surface nodes' 1-based unknowns per axis, [3][n].
+__global__ void green_matrix_kernel(GreenAxis a, GreenAxis b, GreenAxis c, const double* T, const int32_t* u, int n,
+                                    double inv_eps0, double* B) {
+    const GreenAxis ax[3] = {a, b, c};
     const long long total = (long long)n * n;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int i = (int)(t / n), j = (int)(t % n);
-        double v;
-        if (i == k && j == k) v = p;
-        else if (i == k) v = rowk[j] * p;
-        else if (j == k) v = -colk[i] * p;
-        else v = A[t] - colk[i] * rowk[j] * p;
-        A[t] = v;
+        int diff[3], sum[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int p = u[d * n + i], q = u[d * n + j];
+            diff[d] = abs(p - q);
+            sum[d] = ax[d].span + 1 + p + q - 2 * ax[d].lo;
+        }
+        double v = 0.0;
+        for (int x = 0; x < (a.per ? 1 : 2); ++x)
+            for (int y = 0; y < (b.per ? 1 : 2); ++y)
+                for (int z = 0; z < (c.per ? 1 : 2); ++z) {
+                    const double g = T[((long long)(x ? sum[0] : diff[0]) * b.count + (y ? sum[1] : diff[1])) * c.count +
+                                       (z ? sum[2] : diff[2])];
+                    v += (x + y + z) & 1 ? -g : g;
+                }
+        B[t] = v * inv_eps0;
     }
+}
+
+// Blocked in-place Gauss-Jordan inversion without pivoting, kGj pivots a step:
+// with K the pivots' rows and columns, D = A_KK, the row panel becomes R = D^-1
+// A_K (its own columns D^-1), every other row A_i -= A_iK R (its own columns
+// starting from zero). One pass over the matrix per 32 pivots instead of one per
+// pivot. panel: R into `row`, A_:K into `col` ([n][kGj]); every CTA inverts D.
+constexpr int kGj = 32, kGjTile = 64;
+__global__ void __launch_bounds__(256) gj_panel_kernel(const double* A, int n, int k0, double* row, double* col,
+                                                       unsigned* bad) {
+    __shared__ double D[kGj][kGj + 1], pivot_row[kGj], pivot_col[kGj];
+    const int nb = min(kGj, n - k0), tid = threadIdx.x;
+    for (int t = tid; t < kGj * kGj; t += 256) {
+        const int i = t / kGj, j = t % kGj;
+        D[i][j] = i < nb && j < nb ? A[(long long)(k0 + i) * n + k0 + j] : (i == j ? 1.0 : 0.0);
+    }
+    __syncthreads();
+    for (int k = 0; k < nb; ++k) {
+        if (tid < kGj) { pivot_row[tid] = D[k][tid]; pivot_col[tid] = D[tid][k]; }
+        __syncthreads();
+        const double akk = pivot_row[k], p = 1.0 / akk;
+        if (blockIdx.x == 0 && tid == 0 && !(akk > 0.0)) atomicOr(bad, 1u);
+        for (int t = tid; t < kGj * kGj; t += 256) {
+            const int i = t / kGj, j = t % kGj;
+            D[i][j] = i == k ? (j == k ? p : pivot_row[j] * p)
+                             : (j == k ? -pivot_col[i] * p : D[i][j] - pivot_col[i] * pivot_row[j] * p);
+        }
+        __syncthreads();
+    }
+    for (int j = blockIdx.x * 256 + tid; j < n; j += gridDim.x * 256) {
+        double a[kGj];
+#pragma unroll
+        for (int q = 0; q < kGj; ++q) a[q] = q < nb ? A[(long long)(k0 + q) * n + j] : 0.0;
+        const int own = j - k0;
+        for (int i = 0; i < nb; ++i) {
+            double s = 0.0;
+#pragma unroll
+            for (int q = 0; q < kGj; ++q) s += D[i][q] * a[q];
+            row[(long long)i * n + j] = own >= 0 && own < nb ? D[i][own] : s;
+        }
+#pragma unroll
+        for (int q = 0; q < kGj; ++q) col[(long long)j * kGj + q] = q < nb ? A[(long long)j * n + k0 + q] : 0.0;
+    }
+}
+__global__ void __launch_bounds__(256) gj_update_kernel(double* A, int n, int k0, const double* row, const double* col) {
+    __shared__ double R[kGj][kGjTile], C[kGjTile][kGj + 1];
+    const int nb = min(kGj, n - k0), tid = threadIdx.x;
+    const int i0 = blockIdx.y * kGjTile, j0 = blockIdx.x * kGjTile;
+    for (int t = tid; t < kGj * kGjTile; t += 256) {
+        const int q = t / kGjTile, j = j0 + t % kGjTile;
+        R[q][t % kGjTile] = q < nb && j < n ? row[(long long)q * n + j] : 0.0;
+        const int i = i0 + t / kGj;
+        C[t / kGj][t % kGj] = i < n ? col[(long long)i * kGj + t % kGj] : 0.0;
+    }
+    __syncthreads();
+    const int tx = tid & 15, ty = tid >> 4;   // columns tx + 16 q, rows ty + 16 p
+    double s[4][4] = {};
+    for (int q = 0; q < nb; ++q) {
+        double c[4], r[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { c[e] = C[ty + 16 * e][q]; r[e] = R[q][tx + 16 * e]; }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int y = 0; y < 4; ++y) s[x][y] += c[x] * r[y];
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+            const int i = i0 + ty + 16 * x, j = j0 + tx + 16 * y;
+            if (i >= n || j >= n) continue;
+            double* v = A + (long long)i * n + j;
+            if (i >= k0 && i < k0 + nb) *v = R[i - k0][tx + 16 * y];
+            else *v = (j >= k0 && j < k0 + nb ? 0.0 : *v) - s[x][y];
+        }
 }
 
 // colsum_j = sum_i C_ij; scal[3] = sum_ij C_ij (Cmatrix::total, Cmatrix.hpp:36-44).
@@ -343,12 +497,65 @@ static void finish_C(Ctx& c, ObjectDev& o) {
     }
 }
 
-void cmatrix_build(Ctx& c, int id) {
-    ObjectDev& o = c.objs[id];
+// B of an object whose surface nodes are all unknowns of the Poisson solve;
+// false where one is not (it lies on a face or beyond) or the table would not fit.
+static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
+    const MGLevel& m = c.mg[0];
+    GreenAxis ax[3];
+    std::vector<int32_t> u(3 * (size_t)o.n);
+    for (int d = 0; d < 3; ++d) {
+        const int first = m.per[d] ? 1 : 2;   // glue index of the first unknown
+        int lo = 1 << 30, hi = 0;
+        for (int t = 0; t < o.n; ++t) {
+            const int q = o.nodes_ijk[3 * (size_t)t + d] - first + 1;
+            if (q < 1 || q > m.n[d]) return false;
+            u[(size_t)d * o.n + t] = q;
+            lo = std::min(lo, q);
+            hi = std::max(hi, q);
+        }
+        const int span = hi - lo;
+        ax[d] = GreenAxis{m.n[d], m.per[d], lo, span, m.per[d] ? span + 1 : 3 * span + 2, nullptr, nullptr};
+    }
+    const size_t first = (size_t)ax[0].n * ax[1].n * ax[2].count, second = (size_t)ax[0].n * ax[1].count * ax[2].count;
+    const size_t third = (size_t)ax[0].count * ax[1].count * ax[2].count;
+    size_t tables = 0;
+    for (const auto& x : ax) tables += (size_t)x.n * (x.count + 1);
+    const size_t doubles = tables + first + second + third;
+    if (doubles > (size_t)1 << 29) return false;   // 4 GiB
+    double* pool = nullptr;
+    int32_t* du = nullptr;
+    FOPIS_CUDA(cudaMallocAsync((void**)&pool, sizeof(double) * doubles, c.st));
+    FOPIS_CUDA(cudaMallocAsync((void**)&du, sizeof(int32_t) * u.size(), c.st));
+    FOPIS_CUDA(cudaMemcpyAsync(du, u.data(), sizeof(int32_t) * u.size(), cudaMemcpyHostToDevice, c.st));
+    double* next = pool;
+    for (auto& x : ax) {
+        x.cosines = next;
+        x.lambda = next + (size_t)x.n * x.count;
+        next = x.lambda + x.n;
+        ++c.launches;
+        green_axis_kernel<<<grid1((long long)x.n * x.count), kT, 0, c.st>>>(x);
+    }
+    double *R1 = next, *R2 = R1 + first, *T = R2 + second;
+    c.launches += 4;
+    green_sum_kernel<<<dim3((ax[1].n + kGreenL - 1) / kGreenL, ax[0].n), kGreenThreads, sizeof(double) * kGreenL * ax[2].n,
+                       c.st>>>(ax[0], ax[1], ax[2], R1);
+    auto contract = [&](const GreenAxis& x, const double* in, int inner, int outer, double* out) {
+        green_contract_kernel<<<dim3((inner + kGreenThreads - 1) / kGreenThreads, (x.count + kGreenU - 1) / kGreenU, outer),
+                                kGreenThreads, 0, c.st>>>(x, in, inner, out);
+    };
+    contract(ax[1], R1, ax[2].count, ax[0].n, R2);
+    contract(ax[0], R2, ax[1].count * ax[2].count, 1, T);
+    green_matrix_kernel<<<grid1((long long)o.n * o.n), kT, 0, c.st>>>(ax[0], ax[1], ax[2], T, du, o.n, 1.0 / c.p.eps0, B);
+    FOPIS_LAUNCH_CHECK();
+    FOPIS_CUDA(cudaFreeAsync(pool, c.st));
+    FOPIS_CUDA(cudaFreeAsync(du, c.st));
+    FOPIS_CUDA(cudaStreamSynchronize(c.st));   // the node list is a local
+    return true;
+}
+
+// B column by column: one solve per surface node.
+static void solved_matrix(Ctx& c, const ObjectDev& o, double* B) {
     const int n = o.n;
-    double* B = o.C;
-    // keep the user's fields: the reference builds C before any particle exists
-    FOPIS_CUDA(cudaMemsetAsync(c.rho0, 0, sizeof(double) * c.N, c.st));
     const double tol = std::min(c.p.poisson_tol > 0 ? c.p.poisson_tol : 1e-8, 1e-10);
     for (int col = 0; col < n; ++col) {
         const long long node = ((long long)o.nodes_ijk[3 * col] * c.cy + o.nodes_ijk[3 * col + 1]) * c.cz + o.nodes_ijk[3 * col + 2];
@@ -364,24 +571,33 @@ void cmatrix_build(Ctx& c, int id) {
         set_node_kernel<<<1, 1, 0, c.st>>>(c.rho0, node, 0.0);
         FOPIS_LAUNCH_CHECK();
     }
+}
+
+void cmatrix_build(Ctx& c, int id) {
+    ObjectDev& o = c.objs[id];
+    const int n = o.n;
+    double* B = o.C;
+    // keep the user's fields: the reference builds C before any particle exists
+    FOPIS_CUDA(cudaMemsetAsync(c.rho0, 0, sizeof(double) * c.N, c.st));
+    if (!green_matrix(c, o, B)) solved_matrix(c, o, B);
     FOPIS_CUDA(cudaMemsetAsync(c.phi, 0, sizeof(double) * c.N, c.st));
-    double* rowk = nullptr;
+    double* row = nullptr;
     unsigned* bad = nullptr;
-    FOPIS_CUDA(cudaMalloc(&rowk, sizeof(double) * 2 * n));
-    FOPIS_CUDA(cudaMalloc(&bad, sizeof(unsigned)));
+    FOPIS_CUDA(cudaMallocAsync((void**)&row, sizeof(double) * 2 * kGj * n, c.st));
+    FOPIS_CUDA(cudaMallocAsync((void**)&bad, sizeof(unsigned), c.st));
     FOPIS_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned), c.st));
-    for (int k = 0; k < n; ++k) {
-        ++c.launches;
-        gj_copy_kernel<<<grid1(n), kT, 0, c.st>>>(B, n, k, rowk, rowk + n);
-        ++c.launches;
-        gj_update_kernel<<<grid1((long long)n * n), kT, 0, c.st>>>(B, n, k, rowk, rowk + n, bad);
+    const int tiles = (n + kGjTile - 1) / kGjTile;
+    for (int k = 0; k < n; k += kGj) {
+        c.launches += 2;
+        gj_panel_kernel<<<(n + 255) / 256, 256, 0, c.st>>>(B, n, k, row, row + (size_t)kGj * n, bad);
+        gj_update_kernel<<<dim3(tiles, tiles), 256, 0, c.st>>>(B, n, k, row, row + (size_t)kGj * n);
     }
     FOPIS_LAUNCH_CHECK();
     unsigned hbad = 0;
     FOPIS_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, c.st));
+    FOPIS_CUDA(cudaFreeAsync(row, c.st));
+    FOPIS_CUDA(cudaFreeAsync(bad, c.st));
     FOPIS_CUDA(cudaStreamSynchronize(c.st));
-    cudaFree(rowk);
-    cudaFree(bad);
     if (hbad) throw ApiError{FOPIS_ERR_DEVICE, "capacity matrix B is not positive definite"};
     finish_C(c, o);
 }
