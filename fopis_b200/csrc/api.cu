@@ -298,6 +298,7 @@ int fopis_create(const fopis_params* p, int device, void** out) {
     *out = nullptr;
     Ctx* c = new (std::nothrow) Ctx();
     if (!c) return FOPIS_ERR_NOMEM;
+    hostcopy_open();
     int rc = guarded(c, [&](Ctx& x) -> int {
         x.p = *p;
         if (p->nx < 3 || p->ny < 3 || p->nz < 3 || p->nx > 1020 || p->ny > 1020 || p->nz > 1020)
@@ -436,6 +437,7 @@ void fopis_destroy(void* h) {
     for (void* q : ptrs) if (q) cudaFree(q);
     if (c->h_sc) cudaFreeHost(c->h_sc);
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);
+    hostcopy_close(*c);
     if (c->st) cudaStreamDestroy(c->st);
     delete c;
 }
@@ -478,7 +480,7 @@ int fopis_get_capacity_matrix(void* h, int id, double* C, int n) {
     return guarded(h, [&](Ctx& c) -> int {
         if (id < 0 || id >= (int)c.objs.size() || !C || n != c.objs[id].n) throw ApiError{FOPIS_ERR_ARG, "object id or size"};
         if (!c.objs[id].has_C) throw ApiError{FOPIS_ERR_STATE, "capacity matrix not built"};
-        FOPIS_CUDA(cudaMemcpy(C, c.objs[id].C, sizeof(double) * (size_t)n * n, cudaMemcpyDeviceToHost));
+        copy_to_host(c, C, c.objs[id].C, sizeof(double) * (size_t)n * n);
         return FOPIS_OK;
     });
 }
@@ -819,18 +821,18 @@ int fopis_set_field(void* h, int which, const double* in, size_t n) {
     return guarded(h, [&](Ctx& c) -> int {
         if (const YeeArr* y = em_array(c, which)) {
             if (!in || n != y->size()) throw ApiError{FOPIS_ERR_ARG, "input size must be the Yee array's element count"};
-            FOPIS_CUDA(cudaMemcpy(y->v, in, sizeof(double) * n, cudaMemcpyHostToDevice));
+            copy_to_device(c, y->v, in, sizeof(double) * n);
             return FOPIS_OK;
         }
         if (c.em.on && which >= FOPIS_FIELD_JX && which <= FOPIS_FIELD_JZ) {
             if (!in || n != field_elements(c, which)) throw ApiError{FOPIS_ERR_ARG, "input size must be the current's element count"};
-            FOPIS_CUDA(cudaMemcpy(c.em.j[which - FOPIS_FIELD_JX], in, sizeof(double) * n, cudaMemcpyHostToDevice));
+            copy_to_device(c, c.em.j[which - FOPIS_FIELD_JX], in, sizeof(double) * n);
             return FOPIS_OK;
         }
         if (!in || n != c.N) throw ApiError{FOPIS_ERR_ARG, "input size must be (nx+2)(ny+2)(nz+2)"};
         double* dst = which == FOPIS_FIELD_PHI ? c.phi : (which == FOPIS_FIELD_RHO0 ? c.rho0 : nullptr);
         if (!dst) throw ApiError{FOPIS_ERR_ARG, "only PHI and RHO0 can be set"};
-        FOPIS_CUDA(cudaMemcpy(dst, in, sizeof(double) * c.N, cudaMemcpyHostToDevice));
+        copy_to_device(c, dst, in, sizeof(double) * c.N);
         return FOPIS_OK;
     });
 }

@@ -606,7 +606,7 @@ void cmatrix_build(Ctx& c, int id) {
 
 void cmatrix_set(Ctx& c, int id, const double* hostC) {
     ObjectDev& o = c.objs[id];
-    FOPIS_CUDA(cudaMemcpy(o.C, hostC, sizeof(double) * (size_t)o.n * o.n, cudaMemcpyHostToDevice));
+    copy_to_device(c, o.C, hostC, sizeof(double) * (size_t)o.n * o.n);
     finish_C(c, o);
 }
 

@@ -553,23 +553,21 @@ const YeeArr* em_array(const Ctx& c, int which) {
 void em_field_export(Ctx& c, int which, double* host) {
     const size_t bytes = sizeof(double) * c.N;
     if (const YeeArr* y = em_array(c, which)) {
-        FOPIS_CUDA(cudaMemcpyAsync(host, y->v, sizeof(double) * y->size(), cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, y->v, sizeof(double) * y->size());
     } else if (which >= FOPIS_FIELD_JX && which <= FOPIS_FIELD_JZ) {
         const int d = which - FOPIS_FIELD_JX;
         const size_t n = (size_t)(c.cx - (d == 0)) * (c.cy - (d == 1)) * (c.cz - (d == 2));
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.em.j[d], sizeof(double) * n, cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.em.j[d], sizeof(double) * n);
     } else if (which >= FOPIS_FIELD_EXREF && which <= FOPIS_FIELD_EZREF) {
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.em.eref + (size_t)(which - FOPIS_FIELD_EXREF) * c.N, bytes,
-                                   cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.em.eref + (size_t)(which - FOPIS_FIELD_EXREF) * c.N, bytes);
     } else if (which >= FOPIS_FIELD_BXREF && which <= FOPIS_FIELD_BZREF) {
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.em.bref + (size_t)(which - FOPIS_FIELD_BXREF) * c.N, bytes,
-                                   cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.em.bref + (size_t)(which - FOPIS_FIELD_BXREF) * c.N, bytes);
     } else if (which >= FOPIS_FIELD_JXREF && which <= FOPIS_FIELD_JZREF) {
         const int d = which - FOPIS_FIELD_JXREF;
         ++c.launches;
         jref_kernel<<<blocks((long long)c.N), kT, 0, c.st>>>(c.em.j[d], d, make_geo(c), c.scratch64, (long long)c.N);
         FOPIS_LAUNCH_CHECK();
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.scratch64, bytes, cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.scratch64, bytes);
     } else {
         throw ApiError{FOPIS_ERR_ARG, "unknown field selector"};
     }

@@ -335,16 +335,16 @@ void field_export(Ctx& c, int which, double* host) {
     const G g = make_g(c);
     const size_t bytes = sizeof(double) * c.N;
     if (which == FOPIS_FIELD_PHI) {
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.phi, bytes, cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.phi, bytes);
     } else if (which == FOPIS_FIELD_RHO0) {
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.rho0, bytes, cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.rho0, bytes);
     } else if (which >= FOPIS_FIELD_EXREF && which <= FOPIS_FIELD_EZREF) {
         double* tmp = nullptr;
         FOPIS_CUDA(cudaMallocAsync(&tmp, 3 * bytes, c.st));
         ++c.launches;
         efield_kernel<float4><<<blocks((long long)c.N), kT, 0, c.st>>>(c.phi, g, nullptr, tmp, tmp + c.N, tmp + 2 * c.N);
         FOPIS_LAUNCH_CHECK();
-        FOPIS_CUDA(cudaMemcpyAsync(host, tmp + (which - FOPIS_FIELD_EXREF) * c.N, bytes, cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, tmp + (which - FOPIS_FIELD_EXREF) * c.N, bytes);
         FOPIS_CUDA(cudaFreeAsync(tmp, c.st));
     } else if (which >= FOPIS_FIELD_RHO_SPECIES && which < FOPIS_FIELD_RHO_SPECIES + c.nsp) {
         const int s = which - FOPIS_FIELD_RHO_SPECIES;
@@ -357,7 +357,7 @@ void field_export(Ctx& c, int which, double* host) {
             convert_species_kernel<<<blocks((long long)c.N), kT, 0, c.st>>>(c.rho_i64 + (size_t)s * c.N, (long long)c.N,
                                                                            scale, c.scratch64);
         FOPIS_LAUNCH_CHECK();
-        FOPIS_CUDA(cudaMemcpyAsync(host, c.scratch64, bytes, cudaMemcpyDeviceToHost, c.st));
+        copy_to_host(c, host, c.scratch64, bytes);
     } else {
         throw ApiError{FOPIS_ERR_ARG, "unknown field selector"};
     }

@@ -318,6 +318,7 @@ struct Ctx {
     double ms_phase[8] = {0};
     cudaEvent_t ev[9] = {nullptr};
     std::string err;
+    cudaEvent_t copy_ev[16] = {nullptr};   // one per slot of the staged host copies
     int64_t launches = 0;            // kernels launched by this context
     // solve history valid (phi_prev, phi_prev2, phi_obj)
     bool hist_ok = false;
@@ -350,6 +351,24 @@ void launch_energy(Ctx& c);
 void sync_scalars(Ctx& c);
 // fields.cu
 void rho_zero(Ctx& c);
+// hostcopy.cu
+struct CopySegment {
+    void* dev;
+    void* host;
+    size_t bytes;
+};
+void hostcopy_open();
+void hostcopy_close(Ctx& c);
+void copy_to_host(Ctx& c, const CopySegment* s, int n);     // in stream order, complete on return
+void copy_to_device(Ctx& c, const CopySegment* s, int n, bool wait = true);
+inline void copy_to_host(Ctx& c, void* host, const void* dev, size_t bytes) {
+    const CopySegment s{const_cast<void*>(dev), host, bytes};
+    copy_to_host(c, &s, 1);
+}
+inline void copy_to_device(Ctx& c, void* dev, const void* host, size_t bytes, bool wait = true) {
+    const CopySegment s{dev, const_cast<void*>(host), bytes};
+    copy_to_device(c, &s, 1, wait);
+}
 void rho_finalize(Ctx& c);
 double species_rho_scale(const Ctx& c, int s);
 void efield_update(Ctx& c);

@@ -2358,7 +2358,7 @@ static void append_aos(Ctx& c, int s, const void* host56, int64_t n) {
     const Grid g = make_grid(c);
     for (int64_t off = 0; off < n; off += chunk) {
         const int64_t m = std::min(chunk, n - off);
-        FOPIS_CUDA(cudaMemcpyAsync(d, (const char*)host56 + 56 * off, 56 * m, cudaMemcpyHostToDevice, c.st));
+        copy_to_device(c, d, (const char*)host56 + 56 * off, 56 * m, false);   // waited for below
         ++c.launches;
         load56_kernel<<<grid_for(m), kThreads, 0, c.st>>>(parts<T>(c)[s], c.cap[s], &c.d_sc->count[s], d, m, g, c.d_sc);
         FOPIS_LAUNCH_CHECK();
@@ -2407,7 +2407,7 @@ int64_t particles_export_aos(Ctx& c, int s, void* host56, int64_t cap) {
         const int64_t k = c.fp64 ? export_range<double>(c, s, d, nullptr, lo, hi, dc)
                                  : export_range<float>(c, s, d, nullptr, lo, hi, dc);
         const int64_t w = std::max<int64_t>(0, std::min(k, cap - total));
-        if (w > 0) FOPIS_CUDA(cudaMemcpy((char*)host56 + 56 * total, d, 56 * w, cudaMemcpyDeviceToHost));
+        if (w > 0) copy_to_host(c, (char*)host56 + 56 * total, d, 56 * w);
         total += k;
     }
     cudaFree(d);
