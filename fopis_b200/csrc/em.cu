@@ -188,23 +188,35 @@ __global__ void __launch_bounds__(kFdtdK * kFdtdJ) fdtd_b_kernel(Yee bx, Yee by,
     }
 }
 
-// Communicator::sendRecvFieldX/Y/Z self branch (Communicator.cpp:265-343) on a
-// Yee array along one periodic axis (index base 0 there): index 0 <- index
-// m-2, index m-1 <- index 1, over the whole extent of the other two axes.
-__global__ void yee_glue_kernel(Yee a, int n0, int axis) {
-    const int n[3] = {n0, a.n1, a.n2};
-    const int lo[3] = {a.lo0, a.lo1, a.lo2};
-    const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
-    const long long plane = (long long)n[a1] * n[a2];
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < plane; t += (long long)gridDim.x * blockDim.x) {
-        int p[3];
-        p[a1] = lo[a1] + (int)(t / n[a2]);
-        p[a2] = lo[a2] + (int)(t % n[a2]);
-        const int m = n[axis];
-        p[axis] = 1; const double v1 = a.at(p[0], p[1], p[2]);
-        p[axis] = m - 2; const double vm2 = a.at(p[0], p[1], p[2]);
-        p[axis] = 0; a.at(p[0], p[1], p[2]) = vm2;
-        p[axis] = m - 1; a.at(p[0], p[1], p[2]) = v1;
+// Communicator::sendRecvFieldX/Y/Z self branch (Communicator.cpp:265-343) on
+// three Yee arrays along every periodic axis (index base 0 there): index 0 <-
+// index m-2, index m-1 <- index 1, over the whole extent of the other two axes,
+// axis after axis. In one launch: a glue point takes the point with all its
+// periodic indices mapped, which nothing here writes (points on two planes are
+// written twice, alike). A launch per array and axis, nine of a few us each,
+// were most of an update of a small box.
+struct GluePlanes {
+    Yee a[3];
+    int n0[3];
+    int per[3];
+    int n;                     // planes
+    int array[18], axis[18], side[18];
+    long long start[19];
+};
+__global__ void yee_glue_kernel(GluePlanes G) {
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < G.start[G.n]; t += (long long)gridDim.x * blockDim.x) {
+        int q = 0;
+        while (t >= G.start[q + 1]) ++q;
+        const Yee& a = G.a[G.array[q]];
+        const int n[3] = {G.n0[G.array[q]], a.n1, a.n2}, lo[3] = {a.lo0, a.lo1, a.lo2};
+        const int axis = G.axis[q], a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
+        const int r = (int)(t - G.start[q]);
+        int p[3], s[3];
+        p[a1] = lo[a1] + r / n[a2];
+        p[a2] = lo[a2] + r % n[a2];
+        p[axis] = G.side[q] ? n[axis] - 1 : 0;
+        for (int d = 0; d < 3; ++d) s[d] = !G.per[d] ? p[d] : (p[d] == 0 ? n[d] - 2 : (p[d] == n[d] - 1 ? 1 : p[d]));
+        a.at(p[0], p[1], p[2]) = a.at(s[0], s[1], s[2]);
     }
 }
 
@@ -372,15 +384,21 @@ __global__ void em_sum_kernel(const double* partial, int n, double* out) {
     if (threadIdx.x == 0) *out = v;
 }
 
-void yee_glue(Ctx& c, const YeeArr& a) {
-    for (int axis = 0; axis < 3; ++axis) {
-        if (!c.per[2 * axis]) continue;
-        const long long plane = axis == 0 ? (long long)a.n[1] * a.n[2]
-                                          : (axis == 1 ? (long long)a.n[0] * a.n[2] : (long long)a.n[0] * a.n[1]);
-        ++c.launches;
-        yee_glue_kernel<<<blocks(plane), kT, 0, c.st>>>(view(a), a.n[0], axis);
-        FOPIS_LAUNCH_CHECK();
-    }
+// The glue copies of the three arrays from f on.
+void yee_glue(Ctx& c, const YeeArr* f) {
+    GluePlanes G{};
+    for (int q = 0; q < 3; ++q) { G.a[q] = view(f[q]); G.n0[q] = f[q].n[0]; G.per[q] = c.per[2 * q]; }
+    for (int q = 0; q < 3; ++q)
+        for (int axis = 0; axis < 3; ++axis)
+            for (int side = 0; side < 2 && c.per[2 * axis]; ++side) {
+                G.array[G.n] = q; G.axis[G.n] = axis; G.side[G.n] = side;
+                G.start[G.n + 1] = G.start[G.n] + (long long)f[q].size() / f[q].n[axis];
+                ++G.n;
+            }
+    if (G.n == 0) return;
+    ++c.launches;
+    yee_glue_kernel<<<blocks(G.start[G.n]), kT, 0, c.st>>>(G);
+    FOPIS_LAUNCH_CHECK();
 }
 
 void reference_efield(Ctx& c) {
@@ -522,7 +540,7 @@ void em_update_efield(Ctx& c) {
     fdtd_e_kernel<<<fdtd_grid(g), dim3(kFdtdK, kFdtdJ), 0, c.st>>>(view(f[0]), view(f[1]), view(f[2]), view(f[3]), view(f[4]),
                                                               view(f[5]), c.em.j[0], c.em.j[1], c.em.j[2], g, dte, C);
     FOPIS_LAUNCH_CHECK();
-    for (int q = 0; q < 3; ++q) yee_glue(c, f[q]);
+    yee_glue(c, f);
     reference_efield(c);
 }
 
@@ -533,7 +551,7 @@ void em_update_bfield(Ctx& c) {
     fdtd_b_kernel<<<fdtd_grid(g), dim3(kFdtdK, kFdtdJ), 0, c.st>>>(view(f[3]), view(f[4]), view(f[5]), view(f[0]), view(f[1]),
                                                               view(f[2]), g, 1.0 /* dt / dx */);
     FOPIS_LAUNCH_CHECK();
-    for (int q = 3; q < 6; ++q) yee_glue(c, f[q]);
+    yee_glue(c, f + 3);
     reference_bfield(c);
 }
 
@@ -571,7 +589,6 @@ void em_field_export(Ctx& c, int which, double* host) {
     } else {
         throw ApiError{FOPIS_ERR_ARG, "unknown field selector"};
     }
-    FOPIS_CUDA(cudaStreamSynchronize(c.st));
 }
 
 }  // namespace fopis

@@ -30,38 +30,10 @@ int blocks(long long n) {
     return (int)(b < 148LL * 32 ? (b < 1 ? 1 : b) : 148LL * 32);
 }
 
-// Periodic fold of one axis for every species array (integer, exact):
-// MPIw::Environment::sendRecvNodeScalar self-exchange, glue size 2
-// (src/MPI/Communicator.cpp:497-574): node 0 and node n both become their sum,
-// node 1 and node n+1 likewise.
 // A fixed-point fold sum that passed 2^64 (unsigned wrap) is latched as
 // FOPIS_DEV_RHO_OVERFLOW; FP64 sums have no such limit.
 __device__ __forceinline__ bool fold_wrapped(unsigned long long sum, unsigned long long a) { return sum < a; }
 __device__ __forceinline__ bool fold_wrapped(double, double) { return false; }
-
-template <typename W>
-__global__ void fold_kernel(W* rho, int nsp, long long N, G g, int axis, unsigned* status) {
-    const int dims[3] = {g.cx, g.cy, g.cz};
-    const int a1 = axis == 0 ? 1 : 0, a2 = axis == 2 ? 1 : 2;
-    const long long plane = (long long)dims[a1] * dims[a2];
-    const long long total = plane * nsp;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-        const int s = (int)(t / plane);
-        const long long r = t % plane;
-        int idx[3];
-        idx[a1] = (int)(r / dims[a2]);
-        idx[a2] = (int)(r % dims[a2]);
-        W* a = rho + (long long)s * N;
-        const int X = dims[axis];
-        idx[axis] = 0; const long long p0 = L(g, idx[0], idx[1], idx[2]);
-        idx[axis] = X - 2; const long long pn = L(g, idx[0], idx[1], idx[2]);
-        idx[axis] = 1; const long long p1 = L(g, idx[0], idx[1], idx[2]);
-        idx[axis] = X - 1; const long long pn1 = L(g, idx[0], idx[1], idx[2]);
-        const W s0 = a[p0] + a[pn], s1 = a[p1] + a[pn1];
-        if (fold_wrapped(s0, a[p0]) || fold_wrapped(s1, a[p1])) atomicOr(status, (unsigned)FOPIS_DEV_RHO_OVERFLOW);
-        a[p0] = s0; a[pn] = s0; a[p1] = s1; a[pn1] = s1;
-    }
-}
 
 struct Scales { double v[FOPIS_MAX_SPECIES]; };
 
@@ -71,13 +43,55 @@ struct Scales { double v[FOPIS_MAX_SPECIES]; };
 __device__ __forceinline__ double weight_value(unsigned long long w) { return (double)w; }
 __device__ __forceinline__ double weight_value(double w) { return w; }
 
-// rho[0] = sum_s q_s size_s W_s (x 2^-51 in fixed point) (RootGridField.cpp:1206-1214).
+// rho[0] = sum_s q_s size_s W_s (x 2^-51 in fixed point) (RootGridField.cpp:1206-1214),
+// with the periodic folds of every species array before it
+// (MPIw::Environment::sendRecvNodeScalar self-exchange, glue size 2,
+// src/MPI/Communicator.cpp:497-574, axis after axis): along a periodic axis nodes
+// 0 and n both become their sum, nodes 1 and n+1 likewise. A thread takes one
+// class of nodes that the folds join (1, 2, 4 or 8 of them; along a periodic axis
+// class 0 is {0, n}, class 1 is {1, n+1}, the rest single), sums it in the order
+// of the axes and writes all of it, so one launch does what one per axis and the
+// conversion did.
 template <typename W>
-__global__ void convert_kernel(const W* rho, int nsp, long long N, Scales sc, double* rho0) {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < N; t += (long long)gridDim.x * blockDim.x) {
-        double r = 0.0;
-        for (int s = 0; s < nsp; ++s) r += sc.v[s] * weight_value(rho[(long long)s * N + t]);
-        rho0[t] = r;
+__global__ void convert_kernel(W* rho, int nsp, long long N, G g, Scales sc, double* rho0, unsigned* status) {
+    const int m[3] = {g.per[0] ? g.cx - 2 : g.cx, g.per[2] ? g.cy - 2 : g.cy, g.per[4] ? g.cz - 2 : g.cz};
+    const long long total = (long long)m[0] * m[1] * m[2];
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+        const unsigned u = (unsigned)t;   // fewer than 2^31 nodes
+        const int k = (int)(u % (unsigned)m[2]), r = (int)(u / (unsigned)m[2]), j = r % m[1], i = r / m[1];
+        const long long p = L(g, i, j, k);
+        // distance to the joined node along each axis, 0 where there is none
+        const long long dx = g.per[0] && i < 2 ? (long long)(g.cx - 2) * g.cy * g.cz : 0,
+                        dy = g.per[2] && j < 2 ? (long long)(g.cy - 2) * g.cz : 0, dz = g.per[4] && k < 2 ? g.cz - 2 : 0;
+        double v = 0.0;
+        if (dx == 0 && dy == 0 && dz == 0) {
+            for (int s = 0; s < nsp; ++s) v += sc.v[s] * weight_value(rho[(long long)s * N + p]);
+            rho0[p] = v;
+            continue;
+        }
+        for (int s = 0; s < nsp; ++s) {
+            W* a = rho + (long long)s * N + p;
+            bool wrapped = false;
+            auto add = [&](W x, W y) { const W z = x + y; wrapped = wrapped || fold_wrapped(z, x); return z; };
+            W sum = 0;
+            for (int z = 0; z < (dz ? 2 : 1); ++z) {
+                W w = 0;
+                for (int y = 0; y < (dy ? 2 : 1); ++y) {
+                    W x = a[z * dz + y * dy];
+                    if (dx) x = add(x, a[z * dz + y * dy + dx]);
+                    w = y ? add(w, x) : x;
+                }
+                sum = z ? add(sum, w) : w;
+            }
+            if (wrapped) atomicOr(status, (unsigned)FOPIS_DEV_RHO_OVERFLOW);
+            for (int q = 0; q < 8; ++q)
+                if ((!(q & 1) || dx) && (!(q & 2) || dy) && (!(q & 4) || dz))
+                    a[((q & 1) ? dx : 0) + ((q & 2) ? dy : 0) + ((q & 4) ? dz : 0)] = sum;
+            v += sc.v[s] * weight_value(sum);
+        }
+        for (int q = 0; q < 8; ++q)
+            if ((!(q & 1) || dx) && (!(q & 2) || dy) && (!(q & 4) || dz))
+                rho0[p + ((q & 1) ? dx : 0) + ((q & 2) ? dy : 0) + ((q & 4) ? dz : 0)] = v;
     }
 }
 
@@ -275,26 +289,15 @@ void glue_copy(Ctx& c, double* a) {
 
 void rho_finalize(Ctx& c) {
     const G g = make_g(c);
-    const long long planes[3] = {(long long)c.cy * c.cz, (long long)c.cx * c.cz, (long long)c.cx * c.cy};
-    for (int axis = 0; axis < 3; ++axis) {
-        if (!c.per[2 * axis]) continue;
-        ++c.launches;
-        if (c.fp64)
-            fold_kernel<<<blocks(planes[axis] * c.nsp), kT, 0, c.st>>>(reinterpret_cast<double*>(c.rho_i64), c.nsp,
-                                                                       (long long)c.N, g, axis, &c.d_sc->status);
-        else
-            fold_kernel<<<blocks(planes[axis] * c.nsp), kT, 0, c.st>>>(c.rho_i64, c.nsp, (long long)c.N, g, axis,
-                                                                       &c.d_sc->status);
-        FOPIS_LAUNCH_CHECK();
-    }
     Scales sc{};
     for (int s = 0; s < c.nsp; ++s) sc.v[s] = species_rho_scale(c, s);
     ++c.launches;
     if (c.fp64)
-        convert_kernel<<<blocks((long long)c.N), kT, 0, c.st>>>(reinterpret_cast<const double*>(c.rho_i64), c.nsp,
-                                                                (long long)c.N, sc, c.rho0);
+        convert_kernel<<<blocks((long long)c.N), kT, 0, c.st>>>(reinterpret_cast<double*>(c.rho_i64), c.nsp, (long long)c.N,
+                                                                g, sc, c.rho0, &c.d_sc->status);
     else
-        convert_kernel<<<blocks((long long)c.N), kT, 0, c.st>>>(c.rho_i64, c.nsp, (long long)c.N, sc, c.rho0);
+        convert_kernel<<<blocks((long long)c.N), kT, 0, c.st>>>(c.rho_i64, c.nsp, (long long)c.N, g, sc, c.rho0,
+                                                                &c.d_sc->status);
     FOPIS_LAUNCH_CHECK();
 }
 
@@ -361,7 +364,6 @@ void field_export(Ctx& c, int which, double* host) {
     } else {
         throw ApiError{FOPIS_ERR_ARG, "unknown field selector"};
     }
-    FOPIS_CUDA(cudaStreamSynchronize(c.st));
 }
 
 double efield_energy(Ctx& c) {

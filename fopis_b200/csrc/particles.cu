@@ -725,17 +725,47 @@ __global__ void __launch_bounds__(kThreads) em_tail_kernel(PushArgs a, EdgeFix J
     }
 }
 
-// J_d = sum_s q_s size_s 2^-40 (fixed-point sums), FP64, for the three edge arrays.
+// J_d = sum_s q_s size_s 2^-24 (fixed-point sums), FP64, for the three edge
+// arrays, with the periodic folds of edge_fold_kernel (em.cu): a fold makes both
+// points of a pair their sum, axis after axis, so an edge holds the sum over its
+// partners along every periodic axis, added in that order from the unfolded
+// sums. (A fold launch per array and axis took longer than the conversion.)
 struct FixScales { double v[FOPIS_MAX_SPECIES]; };
-__global__ void em_j_convert_kernel(const unsigned long long* fix, long long per_species, int nsp, FixScales sc,
+// Partner of index i along a periodic axis of extent m: planes 0 and m-1 across
+// the current's direction; 1 with m-1 and 0 with m-2 along it.
+__device__ __forceinline__ int fold_partner(int i, int m, bool along) {
+    if (!along) return i == 0 ? m - 1 : (i == m - 1 ? 0 : -1);
+    return i == 0 ? m - 2 : (i == 1 ? m - 1 : (i == m - 2 ? 0 : (i == m - 1 ? 1 : -1)));
+}
+__global__ void em_j_convert_kernel(const unsigned long long* fix, long long per_species, int nsp, FixScales sc, Grid g,
                                     double* jx, long long nx, double* jy, long long ny, double* jz) {
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < per_species;
          t += (long long)gridDim.x * blockDim.x) {   // the three arrays back to back
         double v = 0.0;
-        for (int s = 0; s < nsp; ++s) v += sc.v[s] * (double)(long long)fix[(long long)s * per_species + t];
-        if (t < nx) jx[t] = v;
-        else if (t < nx + ny) jy[t - nx] = v;
-        else jz[t - nx - ny] = v;
+        const int d = t < nx ? 0 : (t < nx + ny ? 1 : 2);
+        const long long base = d == 0 ? 0 : (d == 1 ? nx : nx + ny);
+        const int m[3] = {g.cx - (d == 0), g.cy - (d == 1), g.cz - (d == 2)};
+        const unsigned u = (unsigned)(t - base);
+        const int k = (int)(u % (unsigned)m[2]), j = (int)(u / (unsigned)m[2] % (unsigned)m[1]),
+                  i = (int)(u / (unsigned)m[2] / (unsigned)m[1]);
+        const int pi = g.per[0] ? fold_partner(i, m[0], d == 0) : -1, pj = g.per[2] ? fold_partner(j, m[1], d == 1) : -1,
+                  pk = g.per[4] ? fold_partner(k, m[2], d == 2) : -1;
+        auto raw = [&](int x, int y, int z) {
+            const long long q = base + ((long long)x * m[1] + y) * m[2] + z;
+            double v = 0.0;
+            for (int s = 0; s < nsp; ++s) v += sc.v[s] * (double)(long long)fix[(long long)s * per_species + q];
+            return v;
+        };
+        for (int z = 0; z < (pk >= 0 ? 2 : 1); ++z) {
+            double w = 0.0;
+            for (int y = 0; y < (pj >= 0 ? 2 : 1); ++y) {
+                double x = raw(i, y ? pj : j, z ? pk : k);
+                if (pi >= 0) x += raw(pi, y ? pj : j, z ? pk : k);
+                w = y ? w + x : x;
+            }
+            v = z ? v + w : w;
+        }
+        (d == 0 ? jx : (d == 1 ? jy : jz))[t - base] = v;
     }
 }
 
@@ -2646,8 +2676,8 @@ void launch_em_move(Ctx& c, bool kick) {
         FOPIS_LAUNCH_CHECK();
     }
     ++c.launches;
-    em_j_convert_kernel<<<grid_for(per), kThreads, 0, c.st>>>(c.em.jfix, per, c.nsp, sc, c.em.j[0], nxe, c.em.j[1], nye,
-                                                              c.em.j[2]);
+    em_j_convert_kernel<<<grid_for(per), kThreads, 0, c.st>>>(c.em.jfix, per, c.nsp, sc, make_grid(c), c.em.j[0], nxe,
+                                                              c.em.j[1], nye, c.em.j[2]);
     FOPIS_LAUNCH_CHECK();
     em_fold_currents(c);
 }
@@ -2669,7 +2699,6 @@ void launch_em_position(Ctx& c) {
         else em_position_kernel<float><<<grid_for(c.cap[s]), kThreads, 0, c.st>>>(push_args<float>(c, s), J, q);
         FOPIS_LAUNCH_CHECK();
     }
-    em_fold_currents(c);
 }
 
 template <typename T>
