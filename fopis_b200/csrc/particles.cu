@@ -741,7 +741,6 @@ __global__ void em_j_convert_kernel(const unsigned long long* fix, long long per
                                     double* jx, long long nx, double* jy, long long ny, double* jz) {
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < per_species;
          t += (long long)gridDim.x * blockDim.x) {   // the three arrays back to back
-        double v = 0.0;
         const int d = t < nx ? 0 : (t < nx + ny ? 1 : 2);
         const long long base = d == 0 ? 0 : (d == 1 ? nx : nx + ny);
         const int m[3] = {g.cx - (d == 0), g.cy - (d == 1), g.cz - (d == 2)};
@@ -756,6 +755,7 @@ __global__ void em_j_convert_kernel(const unsigned long long* fix, long long per
             for (int s = 0; s < nsp; ++s) v += sc.v[s] * (double)(long long)fix[(long long)s * per_species + q];
             return v;
         };
+        double v = 0.0;
         for (int z = 0; z < (pk >= 0 ? 2 : 1); ++z) {
             double w = 0.0;
             for (int y = 0; y < (pj >= 0 ? 2 : 1); ++y) {
@@ -2699,6 +2699,7 @@ void launch_em_position(Ctx& c) {
         else em_position_kernel<float><<<grid_for(c.cap[s]), kThreads, 0, c.st>>>(push_args<float>(c, s), J, q);
         FOPIS_LAUNCH_CHECK();
     }
+    em_fold_currents(c);
 }
 
 template <typename T>
