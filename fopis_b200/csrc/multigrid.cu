@@ -1397,7 +1397,11 @@ void mg_setup(Ctx& c) {
         n.scale = f.scale * 0.25;
         c.mg.push_back(n);
     }
-    c.direct = direct_fits(c.mg[0].n);
+    // The EM mode solves at start-up only, unless it has bodies, and keeps the
+    // V-cycles: from a potential that differs in its last digits a few particles in
+    // 1e8 move to the other side of a cell face within some steps, and a move that
+    // changes its cell puts v^2 of its charge on other edges than one that does not.
+    c.direct = !c.em.on && direct_fits(c.mg[0].n);
     if (c.direct) {
         MGLevel& l = c.mg[0];
         FOPIS_CUDA(cudaMalloc(&l.f, sizeof(float) * l.size()));

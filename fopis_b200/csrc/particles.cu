@@ -1063,15 +1063,18 @@ __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a
 // cells in shared memory and is read back with lanes 32 places apart, i.e. in
 // different cells: four groups of warps take the rho moments and the edges of
 // one direction each (summing runs of same-cell particles in registers first,
-// as the ES pass does, made the warp take the flush at nearly every entry once
-// particles have drifted: 7.0 ms). Moves that change
+// as the ES pass does, makes the warp take the flush at nearly every entry once
+// particles have drifted: a fifth more instructions). Moves that change
 // their cell (a tenth of the electrons) are listed and their two halves added
-// one by one; particles whose cells lie outside the window use global atomics.
+// one by one, and so are the particles whose cells lie outside the window, with
+// global atomics (done where they were met, a few of them cost every warp the
+// whole path: 7.0 instead of 6.15 ms at 128^3, and 0.73 instead of 0.43 ms a step
+// at 32^3 once electrons move 0.35 cells a step).
 // Warp sums and 64-bit global atomics for every particle (em_warp_move_current)
-// took 11.0 ms at 128^3 (1.34e8 particles), this 7.0 (1.07 TB/s of the 56 B a
+// took 11.0 ms at 128^3 (1.34e8 particles), this 6.15 (1.2 TB/s of the 56 B a
 // particle); it is bound by the shared-memory and gather wavefronts (69 % of
 // the LSU data path busy) and the latency of the gather. One low word with a
-// carry instead of two pieces: 7.3. 512 threads, because the tile and the batch
+// carry instead of two pieces: 0.25 ms more. 512 threads, because the tile and the batch
 // leave room for two CTAs per SM.
 constexpr int kEmThreads = 512;
 constexpr int kEmRun = 4 * kBatch / kEmThreads;          // entries per thread of a group
@@ -1083,9 +1086,12 @@ struct EmTile {
     unsigned lo[kEdges], hi[kEdges];                     // edge sums
     float o[3][kBatchPad], v[3][kBatchPad];              // start offsets and velocity
     unsigned cells[kBatchPad];                           // start cell of a move that stays; else none, new and old cell, 10 bits each
-    unsigned short list[kBatch];                         // entries that change their cell
-    int listed[2];                                       // of this batch and the next
+    int was[kBatchPad], now[kBatchPad];                  // strays: packed cells, now -1 once gone, kDeposits if it deposits
+    unsigned short list[kBatch];                         // entries that change their cell from the front, strays from the back
+    int listed[2], strays[2];                            // of this batch and the next
 };
+constexpr int kDeposits = 1 << 30;                       // above a packed cell
+static_assert(2 * (sizeof(EmTile) + 1024 + 512) <= 228 * 1024, "two CTAs per SM");
 static_assert(kEmRun * kEmThreads == 4 * kBatch && 32 % kEmRun == 0, "a run lies in one lane's 32 entries");
 
 // A window cell as x, y, z in 3 + 3 + 4 bits, three of which fit a word; kNoCell is none.
@@ -1112,8 +1118,16 @@ __device__ __forceinline__ void edge_add(EmTile& T, int d, unsigned code, const 
         atomicAdd(T.hi + w + edge_step(d, q), (unsigned)(t[q] >> 16));
     }
 }
-// The four edge terms of one direction of em_terms / em_terms_same: flux and the
-// weights of the other two axes, cross = the product term of a whole move.
+// The four edge terms of one direction, rounded as em_terms_same (a whole move:
+// midpoint, and the product term of the other two axes) and em_terms (a half:
+// flux and the weights of the other two axes) round them.
+__device__ __forceinline__ void edge_half(float flux, float wb, float wc, int t[4]) {
+    const float s = kCurrentScale * flux;
+    t[0] = __float2int_rn(s * (1.0f - wb) * (1.0f - wc));
+    t[1] = __float2int_rn(s * wb * (1.0f - wc));
+    t[2] = __float2int_rn(s * (1.0f - wb) * wc);
+    t[3] = __float2int_rn(s * wb * wc);
+}
 __device__ __forceinline__ void edge_terms(float flux, float wb, float wc, float cross, int t[4]) {
     const float s = kCurrentScale * flux;
     t[0] = __float2int_rn(s * ((1.0f - wb) * (1.0f - wc) + cross));
@@ -1122,48 +1136,57 @@ __device__ __forceinline__ void edge_terms(float flux, float wb, float wc, float
     t[3] = __float2int_rn(s * (wb * wc + cross));
 }
 
-// The two halves of a cell-changing move on the edges of direction d.
-__device__ __forceinline__ void edge_cross(EmTile& T, int entry, int d) {
-    const unsigned cells = T.cells[entry];
+// One half of a cell-changing move: the old cell's (fresh 0) or the new one's.
+__device__ __forceinline__ void edge_cross(EmTile& T, int entry, int fresh) {
+    const unsigned cells = T.cells[entry], code = fresh ? (cells >> 10) & kNoCell : cells >> 20;
+    if (code == kNoCell) return;
     PState st{0, 0, 0, T.o[0][entry], T.o[1][entry], T.o[2][entry], T.v[0][entry], T.v[1][entry], T.v[2][entry]};
     float f[3], w[3];
-    int t[4];
-    em_half_old(st, f, w);
-    const int b = d == 0 ? 1 : 0, c = d == 2 ? 1 : 2;
-    edge_terms(f[d], w[b], w[c], 0.0f, t);
-    edge_add(T, d, cells >> 20, t);
-    const unsigned fresh = (cells >> 10) & kNoCell;
-    if (fresh == kNoCell) return;
-    st.ox += st.vx; st.oy += st.vy; st.oz += st.vz;
-    st.ox -= floorf(st.ox); st.oy -= floorf(st.oy); st.oz -= floorf(st.oz);
-    em_half_new(st, f, w);
-    edge_terms(f[d], w[b], w[c], 0.0f, t);
-    edge_add(T, d, fresh, t);
+    if (fresh) {
+        st.ox += st.vx; st.oy += st.vy; st.oz += st.vz;
+        st.ox -= floorf(st.ox); st.oy -= floorf(st.oy); st.oz -= floorf(st.oz);
+        em_half_new(st, f, w);
+    } else {
+        em_half_old(st, f, w);
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        int t[4];
+        edge_half(f[d], w[d == 0 ? 1 : 0], w[d == 2 ? 1 : 2], t);
+        edge_add(T, d, code, t);
+    }
 }
 
-// A particle's current with global atomics, both halves.
-__device__ __noinline__ void em_lane_current(const EdgeFix& J, int oi, int oj, int ok, float ox, float oy, float oz,
-                                             const PState& st, bool live) {
-    const float v[3] = {st.vx, st.vy, st.vz}, o0[3] = {ox, oy, oz};
+// A particle whose start or end lies outside the window, with global atomics:
+// part 0 the whole move or its old cell's half, part 1 the new cell's half, part
+// 2 the charge. Returns true when a node sum wrapped past 2^64.
+__device__ __forceinline__ bool stray_part(const EmTile& T, const PushArgs& a, const EdgeFix& J, int entry, int part) {
+    const int was = T.was[entry], now = T.now[entry] & ~kDeposits;
+    PState st{0, 0, 0, T.o[0][entry], T.o[1][entry], T.o[2][entry], T.v[0][entry], T.v[1][entry], T.v[2][entry]};
+    if (part > 0) {
+        if (T.now[entry] < 0 || (part == 1 && now == was) || (part == 2 && !(T.now[entry] & kDeposits))) return false;
+        st.ox += st.vx; st.oy += st.vy; st.oz += st.vz;
+        st.ox -= floorf(st.ox); st.oy -= floorf(st.oy); st.oz -= floorf(st.oz);
+    }
+    int i, j, k;
+    unpack_cell(part > 0 ? now : was, i, j, k);
+    if (part == 2)
+        return global_deposit(a.rho, a.g, lin(a.g, i, j, k), (unsigned)__float2int_rn(st.ox * kDepositScale),
+                              (unsigned)__float2int_rn(st.oy * kDepositScale), (unsigned)__float2int_rn(st.oz * kDepositScale));
     int t[12];
-    if (live && st.i == oi && st.j == oj && st.k == ok) {
-        em_terms_same(o0, v, t);
-        live = false;
+    if (part == 0 && T.now[entry] >= 0 && now == was) {
+        const float o[3] = {st.ox, st.oy, st.oz}, v[3] = {st.vx, st.vy, st.vz};
+        em_terms_same(o, v, t);
     } else {
-        PState s0 = st;
-        s0.ox = ox; s0.oy = oy; s0.oz = oz;
         float f[3], w[3];
-        em_half_old(s0, f, w);
+        if (part == 0) em_half_old(st, f, w);
+        else em_half_new(st, f, w);
         em_terms(f, w, t);
     }
+#pragma unroll
     for (int q = 0; q < 12; ++q)
-        if (t[q]) atomicAdd(em_term_ptr(J, oi, oj, ok, q), (unsigned long long)(long long)t[q]);
-    if (!live) return;
-    float f[3], w[3];
-    em_half_new(st, f, w);
-    em_terms(f, w, t);
-    for (int q = 0; q < 12; ++q)
-        if (t[q]) atomicAdd(em_term_ptr(J, st.i, st.j, st.k, q), (unsigned long long)(long long)t[q]);
+        if (t[q]) atomicAdd(em_term_ptr(J, i, j, k, q), (unsigned long long)(long long)t[q]);
+    return false;
 }
 
 __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, const int32_t* brick_start, EdgeFix J) {
@@ -1189,7 +1212,7 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
         const long long s1 = min(p1, s0 + (long long)kSegment);
         for (int t = tid; t < kPlanes * kWinCells; t += kEmThreads) T.mom[t] = 0u;
         for (int t = tid; t < kEdges; t += kEmThreads) { T.lo[t] = 0u; T.hi[t] = 0u; }
-        if (tid < 2) T.listed[tid] = 0;
+        if (tid < 2) T.listed[tid] = T.strays[tid] = 0;
         int turn = 0;
         __syncthreads();
         for (long long c0 = s0; c0 < s1; c0 += kBatch, turn ^= 1) {
@@ -1222,7 +1245,6 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
                 // the current: tile entry, listed move, or global atomics
                 const bool tiled = had && oldin && (inwin || !live);
                 const bool crosses = tiled && was != now;
-                if (had && !tiled) em_lane_current(J, oi, oj, ok, ox, oy, oz, st, live);
                 T.cells[e] = !tiled ? kNoCell : (crosses ? kNoCell | now << 10 | was << 20 : was);
                 T.o[0][e] = ox; T.o[1][e] = oy; T.o[2][e] = oz;
                 T.v[0][e] = st.vx; T.v[1][e] = st.vy; T.v[2][e] = st.vz;
@@ -1233,15 +1255,26 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
                     at = __shfl_sync(kFull, at, __ffs(m) - 1);
                     if (crosses) T.list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)e;
                 }
+                const bool moved = live;
                 const bool test = live && (window_body || !inwin);
                 if (__any_sync(kFull, test) && absorb_check(a, st, test)) live = false;
+                const unsigned n = __ballot_sync(kFull, had && !tiled);
+                if (n) {
+                    int at = 0;
+                    if (lane == __ffs(n) - 1) at = atomicAdd(&T.strays[turn], __popc(n));
+                    at = __shfl_sync(kFull, at, __ffs(n) - 1);
+                    if (had && !tiled) {
+                        T.list[kBatch - 1 - (at + __popc(n & ((1u << lane) - 1u)))] = (unsigned short)e;
+                        T.was[e] = cell;
+                        T.now[e] = moved ? pack_cell(st.i, st.j, st.k) | (live ? kDeposits : 0) : -1;
+                    }
+                }
                 const unsigned qa = (unsigned)__float2int_rn(st.ox * kDepositScale);
                 const unsigned qb = (unsigned)__float2int_rn(st.oy * kDepositScale);
                 const unsigned qd = (unsigned)__float2int_rn(st.oz * kDepositScale);
                 T.batch[e] = (live && inwin) ? ((unsigned long long)wc | ((unsigned long long)qa << 10) |
                                                 ((unsigned long long)qb << 28) | ((unsigned long long)qd << 46))
                                              : kNoDeposit;
-                if (live && !inwin) wrap |= global_deposit(a.rho, a.g, lin(a.g, st.i, st.j, st.k), qa, qb, qd);
                 npushed += had;
                 nkept += live;
                 if (had) {
@@ -1278,9 +1311,13 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
                     edge_add(T, group, code, t);
                 }
             }
-            if (tid == 0) T.listed[turn ^ 1] = 0;
-            const int listed = T.listed[turn];
-            for (int t = tid; t < 3 * listed; t += kEmThreads) edge_cross(T, T.list[t / 3], t % 3);
+            if (tid == 0) T.listed[turn ^ 1] = T.strays[turn ^ 1] = 0;
+            const int listed = T.listed[turn], strays = T.strays[turn];
+            for (int t = tid; t < 3 * strays; t += kEmThreads) {
+                const int part = t < strays ? 0 : (t < 2 * strays ? 1 : 2);
+                wrap |= stray_part(T, a, J, T.list[kBatch - 1 - (t - part * strays)], part);
+            }
+            for (int t = tid; t < 2 * listed; t += kEmThreads) edge_cross(T, T.list[t < listed ? t : t - listed], t >= listed);
             __syncthreads();
         }
         wrap |= flush_moments<kEmThreads>(T.mom, reinterpret_cast<unsigned*>(T.batch), a, wx0, wy0, wz0);
