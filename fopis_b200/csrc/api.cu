@@ -431,7 +431,7 @@ void fopis_destroy(void* h) {
         for (void* q : inc) if (q) cudaFree(q);
     }
     mg_free(*c);
-    void* ptrs[] = {c->rho_i64, c->rho0, c->phi, c->phi_prev, c->phi_prev2, c->phi_obj, c->phi_obj2, c->scratch64, c->E, c->E64, c->cellmap,
+    void* ptrs[] = {c->rho_i64, c->rho0, c->phi, c->phi_prev, c->phi_prev2, c->phi_obj, c->phi_obj2, c->scratch64, c->E, c->E64, c->cellmap, c->brick_body,
                     c->node_cmat, c->sort_count, c->sort_offset, c->scan_partials, c->ab.cell, c->ab.ox,
                     c->ab.oy, c->ab.oz, c->ab.vx, c->ab.vy, c->ab.vz, c->ab.species, c->ab.object, c->d_sc};
     for (void* q : ptrs) if (q) cudaFree(q);

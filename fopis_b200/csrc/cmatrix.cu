@@ -415,6 +415,7 @@ void object_upload(Ctx& c, ObjectDev& o, const fopis_object_desc* d, int id) {
     }
     FOPIS_CUDA(cudaMemcpy(c.node_cmat, ncm.data(), sizeof(int32_t) * c.N, cudaMemcpyHostToDevice));
     FOPIS_CUDA(cudaMemcpy(c.cellmap, cmap.data(), c.N, cudaMemcpyHostToDevice));
+    mark_brick_bodies(c);
     FOPIS_CUDA(cudaMalloc(&o.nodes, sizeof(int32_t) * o.n));
     FOPIS_CUDA(cudaMemcpy(o.nodes, lin.data(), sizeof(int32_t) * o.n, cudaMemcpyHostToDevice));
     FOPIS_CUDA(cudaMalloc(&o.C, sizeof(double) * (size_t)o.n * o.n));

@@ -272,6 +272,7 @@ struct Ctx {
     double* scratch64 = nullptr;     // [N] residual / field export
     float4* E = nullptr;             // nodal E (FP32) for the gather
     Vec4d* E64 = nullptr;            // nodal E (FP64) for the gather of the FP64 mode
+    uint8_t* brick_body = nullptr;   // per brick: a body cell in its window
     uint8_t* cellmap = nullptr;      // [N] object id + 1 of the node cell, 0 outside
     int32_t* node_cmat = nullptr;    // [N] (object << 24) | cmat, -1 elsewhere
     // sort
@@ -317,8 +318,8 @@ struct Ctx {
     int learned_used = 0;
     double ms_phase[8] = {0};
     cudaEvent_t ev[9] = {nullptr};
-    std::string err;
     cudaEvent_t copy_ev[16] = {nullptr};   // one per slot of the staged host copies
+    std::string err;
     int64_t launches = 0;            // kernels launched by this context
     // solve history valid (phi_prev, phi_prev2, phi_obj)
     bool hist_ok = false;
@@ -338,6 +339,7 @@ int64_t particles_export_raw(Ctx& c, int s, int32_t* cell, float* ox, float* oy,
 void particles_generate_ambient(Ctx& c);
 void particles_sort(Ctx& c);
 int64_t brick_keys(const Ctx& c);
+void mark_brick_bodies(Ctx& c);
 void launch_push(Ctx& c, bool vel, bool pos, bool dep);
 void launch_deposit_all(Ctx& c);
 void launch_em_velocity(Ctx& c);
@@ -349,8 +351,6 @@ void launch_absorb(Ctx& c);
 void launch_secondary(Ctx& c, bool fused);   // emission of the pending incidents' secondaries
 void launch_energy(Ctx& c);
 void sync_scalars(Ctx& c);
-// fields.cu
-void rho_zero(Ctx& c);
 // hostcopy.cu
 struct CopySegment {
     void* dev;
@@ -369,6 +369,8 @@ inline void copy_to_device(Ctx& c, void* dev, const void* host, size_t bytes, bo
     const CopySegment s{dev, const_cast<void*>(host), bytes};
     copy_to_device(c, &s, 1, wait);
 }
+// fields.cu
+void rho_zero(Ctx& c);
 void rho_finalize(Ctx& c);
 double species_rho_scale(const Ctx& c, int s);
 void efield_update(Ctx& c);

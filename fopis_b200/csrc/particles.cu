@@ -224,6 +224,7 @@ struct PushArgsT {
     T bx, by, bz, boris;      // static B as the reference uses it, 2/(1+|b|^2)
     int bzero;                // B = 0: the rotation adds exact zeros and is skipped
     const uint8_t* cellmap;   // nullptr without objects
+    const uint8_t* brick_body;   // per brick: a body cell in its window (nullptr without objects)
     unsigned long long* rho;  // species accumulator: int64 fixed point, or FP64 weights in the FP64 mode
     AbsorbList ab;
     DevScalars* sc;
@@ -935,6 +936,38 @@ __device__ __forceinline__ bool flush_moments(const unsigned* mom, unsigned* t_l
     return wrap;
 }
 
+// Adds a block's kinetic energy and particle counts to the species' totals.
+template <int THREADS>
+__device__ __forceinline__ void brick_totals(const PushArgs& a, double e2, int npushed, int nkept) {
+    __shared__ double s_e[THREADS / 32];
+    __shared__ int s_n[2][THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int o = 16; o; o >>= 1) e2 += __shfl_down_sync(kFull, e2, o);
+    npushed = __reduce_add_sync(kFull, npushed);
+    nkept = __reduce_add_sync(kFull, nkept);
+    if (lane == 0) { s_e[warp] = e2; s_n[0][warp] = npushed; s_n[1][warp] = nkept; }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < THREADS / 32; ++w) { e2 += s_e[w]; npushed += s_n[0][w]; nkept += s_n[1][w]; }
+    if (e2 != 0.0) atomicAdd(&a.sc->energy[a.s], e2);
+    if (npushed > 0) atomicAdd(&a.sc->pushed[a.s], (unsigned long long)npushed);
+    if (nkept > 0) atomicAdd(&a.sc->survived[a.s], (unsigned long long)nkept);
+}
+
+// Whether a body cell lies in a brick's window (the brick and its halo), one
+// brick per thread; the bodies of a context only change when one is added.
+__global__ void brick_body_kernel(Grid g, const uint8_t* cellmap, uint8_t* body) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= g.nb[0] * g.nb[1] * g.nb[2]) return;
+    const int bi = b / (g.nb[1] * g.nb[2]), bj = (b / g.nb[2]) % g.nb[1], bk = b % g.nb[2];
+    uint8_t found = 0;
+    for (int x = max(bi * kBX - kHalo, 0); x < min(bi * kBX - kHalo + kCX, g.cx - 1); ++x)
+        for (int y = max(bj * kBY - kHalo, 0); y < min(bj * kBY - kHalo + kCY, g.cy - 1); ++y)
+            for (int z = max(bk * kBZ - kHalo, 0); z < min(bk * kBZ - kHalo + kCZ, g.cz - 1); ++z)
+                found |= cellmap[lin(g, x, y, z)] != 0;
+    body[b] = found;
+}
+
 __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a, const int32_t* brick_start) {
     __shared__ __align__(16) unsigned s_mom[kPlanes * kWinCells];
     __shared__ __align__(16) unsigned long long s_batch[kBatchPad];    // batch entries; node tile in the epilogue
@@ -943,18 +976,27 @@ __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a
     const int b = blockIdx.x;
     const int bi = b / (a.g.nb[1] * a.g.nb[2]), bj = (b / a.g.nb[2]) % a.g.nb[1], bk = b % a.g.nb[2];
     const int wx0 = bi * kBX - kHalo, wy0 = bj * kBY - kHalo, wz0 = bk * kBZ - kHalo;
-    int body = 0;
-    for (int t = tid; t < kWinCells; t += kBrickThreads) {
-        // a body cell anywhere in the window?
-        const int x = wx0 + t / (kCY * kCZ), y = wy0 + (t / kCZ) % kCY, z = wz0 + t % kCZ;
-        if (a.cellmap && x >= 0 && y >= 0 && z >= 0 && x < a.g.cx - 1 && y < a.g.cy - 1 && z < a.g.cz - 1 &&
-            a.cellmap[lin(a.g, x, y, z)] != 0)
-            body = 1;
-    }
-    // particles that stay inside a body-free window need no body test
-    const bool window_body = __syncthreads_or(body) != 0;
     const long long p0 = brick_start[b], p1 = brick_start[b + 1];
-    double e2 = 0.0, npushed = 0.0, nkept = 0.0;
+    if (p0 == p1) return;
+    // particles that stay inside a body-free window need no body test
+    const bool window_body = a.brick_body && a.brick_body[b];
+    double e2 = 0.0;
+    int npushed = 0, nkept = 0;
+    int32_t cell[kPer];
+    float f[kPer][6];
+    auto load = [&](long long cp, long long end) {
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+            const long long idx = cp + (r * (kBrickThreads / 32) + warp) * 32 + lane;
+            cell[r] = idx < end ? a.p.cell[idx] : -1;
+            if (cell[r] >= 0) {
+                f[r][0] = a.p.ox[idx]; f[r][1] = a.p.oy[idx]; f[r][2] = a.p.oz[idx];
+                f[r][3] = a.p.vx[idx]; f[r][4] = a.p.vy[idx]; f[r][5] = a.p.vz[idx];
+            }
+        }
+    };
+    // the first pass' state travels while the moment tile is cleared
+    load(p0, min(p1, p0 + (long long)kSegment));
     bool wrap = false;
     for (long long s0 = p0; s0 < p1; s0 += kSegment) {
         const long long s1 = min(p1, s0 + (long long)kSegment);
@@ -964,18 +1006,7 @@ __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a
         for (long long c0 = s0; c0 < s1; c0 += kBatch) {
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
-                const long long cp = c0 + h * kPass;
-                int32_t cell[kPer];
-                float f[kPer][6];
-#pragma unroll
-                for (int r = 0; r < kPer; ++r) {
-                    const long long idx = cp + (r * (kBrickThreads / 32) + warp) * 32 + lane;
-                    cell[r] = idx < s1 ? a.p.cell[idx] : -1;
-                    if (cell[r] >= 0) {
-                        f[r][0] = a.p.ox[idx]; f[r][1] = a.p.oy[idx]; f[r][2] = a.p.oz[idx];
-                        f[r][3] = a.p.vx[idx]; f[r][4] = a.p.vy[idx]; f[r][5] = a.p.vz[idx];
-                    }
-                }
+                if (h > 0 || c0 > p0) load(c0 + h * kPass, s1);
 #pragma unroll
                 for (int r = 0; r < kPer; ++r) {
                     const int q = h * kPass + (r * (kBrickThreads / 32) + warp) * 32 + lane;   // place in the batch
@@ -1004,8 +1035,8 @@ __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a
                                            : kNoDeposit;
                     if (live && !inwin) wrap |= global_deposit(a.rho, a.g, lin(a.g, st.i, st.j, st.k), qa, qb, qd);
                     if (live) e2 += (double)(st.vx * st.vx + st.vy * st.vy + st.vz * st.vz);
-                    npushed += cell[r] >= 0 ? 1.0 : 0.0;
-                    nkept += live ? 1.0 : 0.0;
+                    npushed += cell[r] >= 0;
+                    nkept += live;
                     if (cell[r] >= 0) {
                         a.p.cell[idx] = live ? pack_cell(st.i, st.j, st.k) : -1;
                         a.p.ox[idx] = st.ox; a.p.oy[idx] = st.oy; a.p.oz[idx] = st.oz;
@@ -1040,13 +1071,7 @@ __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a
         wrap |= flush_moments<kBrickThreads>(s_mom, t_lo, a, wx0, wy0, wz0);
     }
     if (wrap) atomicOr(&a.sc->status, (unsigned)FOPIS_DEV_RHO_OVERFLOW);
-    const double tot = block_sum(e2);
-    if (tid == 0 && tot != 0.0) atomicAdd(&a.sc->energy[a.s], tot);
-    const double np = block_sum(npushed), nk = block_sum(nkept);
-    if (tid == 0) {
-        if (np > 0.0) atomicAdd(&a.sc->pushed[a.s], (unsigned long long)np);
-        if (nk > 0.0) atomicAdd(&a.sc->survived[a.s], (unsigned long long)nk);
-    }
+    brick_totals<kBrickThreads>(a, e2, npushed, nkept);
 }
 
 // ------------------------------------------------------------------ EM brick push
@@ -1198,14 +1223,7 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
     const int wx0 = bi * kBX - kHalo, wy0 = bj * kBY - kHalo, wz0 = bk * kBZ - kHalo;
     const long long p0 = brick_start[b], p1 = brick_start[b + 1];
     if (p0 == p1) return;
-    int body = 0;
-    for (int t = tid; t < kWinCells; t += kEmThreads) {
-        const int x = wx0 + t / (kCY * kCZ), y = wy0 + (t / kCZ) % kCY, z = wz0 + t % kCZ;
-        if (a.cellmap && x >= 0 && y >= 0 && z >= 0 && x < a.g.cx - 1 && y < a.g.cy - 1 && z < a.g.cz - 1 &&
-            a.cellmap[lin(a.g, x, y, z)] != 0)
-            body = 1;
-    }
-    const bool window_body = __syncthreads_or(body) != 0;
+    const bool window_body = a.brick_body && a.brick_body[b];
     int npushed = 0, nkept = 0;
     bool wrap = false;
     for (long long s0 = p0; s0 < p1; s0 += kSegment) {
@@ -1340,11 +1358,7 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
         __syncthreads();
     }
     if (wrap) atomicOr(&a.sc->status, (unsigned)FOPIS_DEV_RHO_OVERFLOW);
-    const double np = block_sum((double)npushed), nk = block_sum((double)nkept);
-    if (tid == 0) {
-        if (np > 0.0) atomicAdd(&a.sc->pushed[a.s], (unsigned long long)np);
-        if (nk > 0.0) atomicAdd(&a.sc->survived[a.s], (unsigned long long)nk);
-    }
+    brick_totals<kEmThreads>(a, 0.0, npushed, nkept);
 }
 
 // Writes a particle created in FP64 into a species slot (split precision).
@@ -2553,6 +2567,15 @@ int brick_count(const Ctx& c) {
     return g.nb[0] * g.nb[1] * g.nb[2];
 }
 
+// After the cell map changed (a body was added).
+void mark_brick_bodies(Ctx& c) {
+    const int n = brick_count(c);
+    if (!c.brick_body) FOPIS_CUDA(cudaMalloc(&c.brick_body, n));
+    ++c.launches;
+    brick_body_kernel<<<(n + kThreads - 1) / kThreads, kThreads, 0, c.st>>>(make_grid(c), c.cellmap, c.brick_body);
+    FOPIS_LAUNCH_CHECK();
+}
+
 // Sort of every species by brick (brick_index), then by cell inside the
 // brick (local_cell); invalid slots are dropped. Records each brick's first slot
 // for push_brick_kernel. The particles end in the live arrays; the sort
@@ -2634,6 +2657,7 @@ static PushArgsT<T> push_args(Ctx& c, int s) {
     a.boris = (T)(2.0 / (1.0 + b2));
     a.bzero = b2 == 0.0 ? 1 : 0;
     a.cellmap = c.objs.empty() ? nullptr : c.cellmap;
+    a.brick_body = c.objs.empty() ? nullptr : c.brick_body;
     a.rho = c.rho_i64 + (size_t)s * c.N;
     a.ab = c.ab; a.sc = c.d_sc;
     return a;
