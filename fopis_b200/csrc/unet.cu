@@ -310,129 +310,125 @@ struct WgArgs {
     unsigned int* err;
 };
 
-__host__ __device__ constexpr int wg_taps_per_mtile(int cin) { return 128 / cin; }
-__host__ __device__ constexpr int wg_mtiles(int cin) { return (27 + 128 / cin - 1) / (128 / cin); }
-__host__ __device__ constexpr int wg_mt_per_cta(int cin, int cout) {
-    return wg_mtiles(cin) < 4 ? (wg_mtiles(cin) < 128 / cout ? wg_mtiles(cin) : 128 / cout)
-                              : (4 < 128 / cout ? 4 : 128 / cout);
-}
 __host__ __device__ constexpr int pow2_cols(int c) { return c <= 32 ? 32 : c <= 64 ? 64 : c <= 128 ? 128 : 256; }
 
 template <int CIN, int COUT>
 struct WgShape {
-    static constexpr int KC = 32, NST = 3, LA = 1;
+    static constexpr int KC = 128, NST = 3, LA = 2;
     static constexpr int PLI = CIN / 8;
-    static constexpr int TPM = wg_taps_per_mtile(CIN);
-    static constexpr int MTILES = wg_mtiles(CIN);
-    static constexpr int MTC = wg_mt_per_cta(CIN, COUT);
-    static constexpr int GRP = KC * 16;
-    static constexpr int A_MT = 16 * GRP;
-    static constexpr int A_BYTES = MTC * A_MT;
-    static constexpr int B_BYTES = (COUT / 8) * GRP;
+    static constexpr int SEG = 9 * PLI;                          // (di, dj, 8-channel plane) segments
+    static constexpr int YSPLIT = (SEG + 15) / 16;               // CTAs sharing them, at most 16 (M = 128) each
+    static constexpr int GPT = (SEG + YSPLIT - 1) / YSPLIT;
+    static constexpr int GRP = (KC + 2) * 16;                    // a segment: KC positions and one more at either end
+    static constexpr int B_PL = KC * 16;
+    static constexpr int A_BYTES = 16 * GRP;
+    static constexpr int B_BYTES = (COUT / 8) * B_PL;
     static constexpr int ST = A_BYTES + B_BYTES;
-    static constexpr int COLS = pow2_cols(MTC * COUT);
-    static constexpr int SMEM = NST * ST + (NST + 1) * 8 + 16;
-    static constexpr int YSPLIT = (MTILES + MTC - 1) / MTC;
+    static constexpr int COLS = pow2_cols(3 * COUT);
+    static constexpr int SMEM = NST * ST + (2 * NST + 1) * 8 + 16;
 };
 
-__device__ __forceinline__ long long tap_offset(int t, long long Si, long long Sj) {
-    return (long long)(t / 9 - 1) * Si + (long long)((t / 3) % 3 - 1) * Sj + (t % 3 - 1);
-}
-
+// A stage holds KC positions of the output gradient's planes and, for up to 16
+// (di, dj, 8-channel plane) segments, KC + 2 positions of the input. With
+// positions as K a segment is consecutive positions of a plane, so it arrives as
+// one contiguous bulk copy (2 KB, TMA engine), a lane of warp 0 issuing each and
+// the stage's full barrier counting their bytes; the three dk taps read it from
+// one position later each, into three accumulators. The six layers of a training
+// step at 63^3 .. 15^3 take 136 us; 16-byte cp.async per tap and position
+// (issue-bound), or a 512-byte bulk copy per tap (copy-rate-bound), 389.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128) wgrad_kernel(WgArgs a) {
     using S = WgShape<CIN, COUT>;
     constexpr uint32_t IDESC = tc::idesc_bf16(128, COUT, true, true);
     extern __shared__ __align__(128) uint8_t sm[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S::NST * S::ST);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bar + S::NST + 1);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S::NST * S::ST);   // [NST] MMAs done, then all done
+    uint64_t* full = bar + S::NST + 1;                                   // [NST] stage data landed
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(full + S::NST);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int mt0 = blockIdx.y * S::MTC;
-    const int nmt = min(S::MTC, S::MTILES - mt0);
-    // A groups of taps beyond 26 (last M-tile only) are never loaded: zero them once
-    for (int bb = 0; bb < S::NST; ++bb)
-        for (int mt = 0; mt < nmt; ++mt)
-            for (int gq = 0; gq < 16; ++gq) {
-                const int t = (mt0 + mt) * S::TPM + gq / S::PLI;
-                if (t < 27) continue;
-                uint4* d = reinterpret_cast<uint4*>(sm + bb * S::ST + mt * S::A_MT + gq * S::GRP);
-                for (int e = tid; e < S::GRP / 16; e += 128) d[e] = make_uint4(0, 0, 0, 0);
-            }
+    const int s0 = blockIdx.y * S::GPT, groups = min(S::GPT, S::SEG - s0);
+    // the groups without a segment stay zero
+    for (int b = 0; b < S::NST; ++b) {
+        uint4* d = reinterpret_cast<uint4*>(sm + b * S::ST + groups * S::GRP);
+        for (int e = tid; e < (16 - groups) * S::GRP / 16; e += 128) d[e] = make_uint4(0, 0, 0, 0);
+    }
     if (warp == 0) tc::tmem_alloc(tc::saddr(tslot), S::COLS);
     if (tid == 0) {
         for (int b = 0; b <= S::NST; ++b) tc::mbar_init(tc::saddr(bar + b), 1);
+        for (int b = 0; b < S::NST; ++b) tc::mbar_init(tc::saddr(full + b), 1);
         tc::fence_mbar_init();
     }
+    tc::fence_async_smem();   // the zeroed groups, before the tensor core reads them
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = *tslot;
     const uint32_t sbase = tc::saddr(sm);
+    const uint32_t stage_tx = (uint32_t)(groups * S::GRP + S::B_BYTES);
     const long long nloc = (long long)blockIdx.x < a.chunks ? (a.chunks - 1 - blockIdx.x) / gridDim.x + 1 : 0;
     float bsum = 0.0f;
     for (long long q = 0; q < nloc + S::LA; ++q) {
-        if (q < nloc) {
+        if (q < nloc && warp == 0) {
             const int b = (int)(q % S::NST);
             if (q >= S::NST && !tc::mbar_wait(tc::saddr(bar + b), (uint32_t)((q / S::NST) - 1) & 1u)) report(a.err, 4u);
             const long long p0 = ((long long)blockIdx.x + q * gridDim.x) * S::KC;
-            const uint32_t sA = sbase + b * S::ST, sB = sA + S::A_BYTES;
-            for (int e = tid; e < nmt * 16 * S::KC; e += 128) {
-                const int mt = e / (16 * S::KC), rem = e - mt * 16 * S::KC;
-                const int gq = rem / S::KC, k = rem - gq * S::KC;
-                const int t = (mt0 + mt) * S::TPM + gq / S::PLI, pl = gq % S::PLI;
-                if (t >= 27) continue;
-                const long long src = p0 + k + tap_offset(t, a.Si, a.Sj);
-                tc::cp16(sA + mt * S::A_MT + gq * S::GRP + k * 16, a.x.p + ((long long)pl * a.x.stride + src) * 8);
-            }
-            for (int e = tid; e < (COUT / 8) * S::KC; e += 128) {
-                const int pl = e / S::KC, k = e - pl * S::KC;
-                tc::cp16(sB + pl * S::GRP + k * 16, a.g.p + ((long long)pl * a.g.stride + p0 + k) * 8);
+            const uint32_t sA = sbase + b * S::ST, sB = sA + S::A_BYTES, fb = tc::saddr(full + b);
+            if (lane == 0) tc::mbar_arrive_expect_tx(fb, stage_tx);
+            __syncwarp();
+            for (int e = lane; e < groups + COUT / 8; e += 32) {
+                if (e < groups) {
+                    const int t = (s0 + e) / S::PLI, pl = (s0 + e) % S::PLI;
+                    const long long src = p0 + (long long)(t / 3 - 1) * a.Si + (long long)(t % 3 - 1) * a.Sj - 1;
+                    tc::bulk_g2s(sA + e * S::GRP, a.x.p + ((long long)pl * a.x.stride + src) * 8, S::GRP, fb);
+                } else {
+                    const int pl = e - groups;
+                    tc::bulk_g2s(sB + pl * S::B_PL, a.g.p + ((long long)pl * a.g.stride + p0) * 8, S::B_PL, fb);
+                }
             }
         }
-        tc::cp_commit();
         const long long cq = q - S::LA;
         if (cq < 0) continue;
-        tc::cp_wait<S::LA>();
-        tc::fence_async_smem();
-        __syncthreads();
         const int b = (int)(cq % S::NST);
+        if (!tc::mbar_wait(tc::saddr(full + b), (uint32_t)(cq / S::NST) & 1u)) report(a.err, 4u);
         const uint32_t sA = sbase + b * S::ST, sB = sA + S::A_BYTES;
         if (tid == 0) {
             tc::fence_after();
-            for (int mt = 0; mt < nmt; ++mt)
+#pragma unroll
+            for (int dk = 0; dk < 3; ++dk)
 #pragma unroll
                 for (int j = 0; j < S::KC / 16; ++j) {
-                    const uint64_t ad = tc::sdesc(sA + mt * S::A_MT + j * 256, 128, S::GRP);
-                    const uint64_t bd = tc::sdesc(sB + j * 256, 128, S::GRP);
-                    tc::mma(tmem + mt * COUT, ad, bd, IDESC, (cq | j) != 0 ? 1u : 0u);
+                    const uint64_t ad = tc::sdesc(sA + dk * 16 + j * 256, 128, S::GRP);
+                    const uint64_t bd = tc::sdesc(sB + j * 256, 128, S::B_PL);
+                    tc::mma(tmem + dk * COUT, ad, bd, IDESC, (cq | j) != 0 ? 1u : 0u);
                 }
             tc::commit(tc::saddr(bar + b));
         }
-        if (blockIdx.y == 0 && tid < COUT) {
-            const bf16* gb = reinterpret_cast<const bf16*>(sm + b * S::ST + S::A_BYTES + (tid / 8) * S::GRP) + (tid % 8);
+        if (blockIdx.y == 0) {   // channel tid % COUT, every (128 / COUT)-th position
+            const int ch = tid % COUT;
+            const bf16* gb = reinterpret_cast<const bf16*>(sm + b * S::ST + S::A_BYTES + (ch / 8) * S::B_PL) + ch % 8;
 #pragma unroll 8
-            for (int k = 0; k < S::KC; ++k) bsum += __bfloat162float(gb[k * 8]);
+            for (int k = tid / COUT; k < S::KC; k += 128 / COUT) bsum += __bfloat162float(gb[k * 8]);
         }
+        __syncthreads();   // the bias sums have read the stage before it is filled again
     }
     if (nloc > 0) {
         if (tid == 0) tc::commit(tc::saddr(bar + S::NST));
         if (!tc::mbar_wait(tc::saddr(bar + S::NST), 0u)) report(a.err, 8u);
         tc::fence_after();
         const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
-        const int m = warp * 32 + lane;
-        for (int mt = 0; mt < nmt; ++mt) {
+        const int m = warp * 32 + lane, seg = s0 + m / 8;
+        for (int dk = 0; dk < 3; ++dk) {
             uint32_t r[COUT];
 #pragma unroll
-            for (int c = 0; c < COUT; c += 16) tc::tmem_ld16(ta + mt * COUT + c, r + c);
+            for (int c = 0; c < COUT; c += 16) tc::tmem_ld16(ta + dk * COUT + c, r + c);
             tc::tmem_wait<COUT>(r);
-            const int t = (mt0 + mt) * S::TPM + m / CIN, ci = m % CIN;
-            if (t < 27) {
+            if (m / 8 < groups) {
+                const int t = seg / S::PLI * 3 + dk, ci = seg % S::PLI * 8 + m % 8;
                 float* dst = a.dw + (size_t)t * COUT * CIN + ci;
 #pragma unroll
                 for (int co = 0; co < COUT; ++co) atomicAdd(dst + (size_t)co * CIN, __uint_as_float(r[co]));
             }
         }
-        if (blockIdx.y == 0 && tid < COUT) atomicAdd(a.db + tid, bsum);
+        if (blockIdx.y == 0) atomicAdd(a.db + tid % COUT, bsum);
     }
     tc::fence_before();
     __syncthreads();
@@ -552,6 +548,17 @@ __global__ void __launch_bounds__(256) feat_write_kernel(FeatArgs F, const doubl
 }
 
 // phi += sigma_d * prediction on the unknowns.
+// The predicted increment in the glue layout (FP64), zero off the unknowns.
+__global__ void __launch_bounds__(256) predict_kernel(FeatArgs F, const float* out, const double* stats, int cx,
+                                                      double* pred) {
+    const long long N = (long long)cx * F.cy * F.cz;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < N; t += (long long)gridDim.x * blockDim.x) {
+        const int c = (int)(t % F.cz) - F.o2, b = (int)(t / F.cz % F.cy) - F.o1, a = (int)(t / F.cz / F.cy) - F.o0;
+        const bool in = a >= 0 && b >= 0 && c >= 0 && a < F.n0 && b < F.n1 && c < F.n2;
+        pred[t] = in ? stats[7] * (double)out[pos_of(F.g, a, b, c)] : 0.0;
+    }
+}
+
 __global__ void __launch_bounds__(256) apply_guess_kernel(FeatArgs F, const float* out, const double* stats,
                                                           double* phi) {
     const double sd = stats[7];
@@ -1260,35 +1267,25 @@ int unet_eval(Ctx& c, const double* rho0, const double* phi1, const double* phi2
         double* d;
         ~Free() { cudaFreeAsync(d, c.st); }
     } guard{c, d};
-    FOPIS_CUDA(cudaMemcpyAsync(d, rho0, bytes, cudaMemcpyHostToDevice, c.st));
-    FOPIS_CUDA(cudaMemcpyAsync(d + c.N, phi1, bytes, cudaMemcpyHostToDevice, c.st));
-    FOPIS_CUDA(cudaMemcpyAsync(d + 2 * c.N, phi2, bytes, cudaMemcpyHostToDevice, c.st));
+    const CopySegment in[4] = {{d, const_cast<double*>(rho0), bytes}, {d + c.N, const_cast<double*>(phi1), bytes},
+                               {d + 2 * c.N, const_cast<double*>(phi2), bytes},
+                               {d + 3 * c.N, const_cast<double*>(phi_target), bytes}};
+    copy_to_device(c, in, phi_target ? 4 : 3, false);   // check_err waits
     forward(c, n, d, d + c.N, d + 2 * c.N);
     n.fwd_valid = false;
-    if (phi_target) {
-        FOPIS_CUDA(cudaMemcpyAsync(d + 3 * c.N, phi_target, bytes, cudaMemcpyHostToDevice, c.st));
-        backward(c, n, d + 3 * c.N, d + c.N);
-    }
+    if (phi_target) backward(c, n, d + 3 * c.N, d + c.N);
     FOPIS_CUDA(cudaMemcpyAsync(n.h_stats, n.stats, 16 * sizeof(double), cudaMemcpyDeviceToHost, c.st));
-    std::vector<float> out(n.G[0].P);
-    FOPIS_CUDA(cudaMemcpyAsync(out.data(), n.out, sizeof(float) * out.size(), cudaMemcpyDeviceToHost, c.st));
     if (grads && phi_target)
         FOPIS_CUDA(cudaMemcpyAsync(grads, n.grad, sizeof(float) * n.nprm, cudaMemcpyDeviceToHost, c.st));
-    check_err(c, n);
-    const double sd = n.h_stats[7];
-    if (loss) *loss = phi_target ? n.h_stats[11] / ((double)c.mg[0].n[0] * c.mg[0].n[1] * c.mg[0].n[2]) : 0.0;
     if (pred) {
-        std::fill(pred, pred + c.N, 0.0);
-        const MGLevel& m = c.mg[0];
-        const int o[3] = {m.per[0] ? 1 : 2, m.per[1] ? 1 : 2, m.per[2] ? 1 : 2};
-        const NGrid& g = n.G[0];
-        for (int a = 0; a < m.n[0]; ++a)
-            for (int b = 0; b < m.n[1]; ++b)
-                for (int k = 0; k < m.n[2]; ++k) {
-                    const long long p = (long long)(a + 1) * g.Si + (long long)(b + 1) * g.Sj + (k + 1);
-                    pred[((size_t)(a + o[0]) * c.cy + (b + o[1])) * c.cz + (k + o[2])] = sd * (double)out[p];
-                }
+        ++c.launches;
+        predict_kernel<<<row_grid(std::min<long long>((long long)c.cx * c.cy, n.sms * 8)), 256, 0, c.st>>>(
+            feat_args(c, n), n.out, n.stats, c.cx, d);   // the features have read rho0
+        FOPIS_LAUNCH_CHECK();
+        copy_to_host(c, pred, d, bytes);
     }
+    check_err(c, n);
+    if (loss) *loss = phi_target ? n.h_stats[11] / ((double)c.mg[0].n[0] * c.mg[0].n[1] * c.mg[0].n[2]) : 0.0;
     return FOPIS_OK;
 }
 
