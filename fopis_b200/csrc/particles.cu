@@ -2740,7 +2740,6 @@ void launch_em_move(Ctx& c, bool kick) {
     em_j_convert_kernel<<<grid_for(per), kThreads, 0, c.st>>>(c.em.jfix, per, c.nsp, sc, make_grid(c), c.em.j[0], nxe,
                                                               c.em.j[1], nye, c.em.j[2]);
     FOPIS_LAUNCH_CHECK();
-    em_fold_currents(c);
 }
 
 // RootGrid::updateParticlePositionEM: J = 0 (Field::initializeCurrent), the
