@@ -501,7 +501,7 @@ static void finish_C(Ctx& c, ObjectDev& o) {
 }
 
 // B of an object whose surface nodes are all unknowns of the Poisson solve;
-// false where one is not (it lies on a face or beyond) or the table would not fit.
+// false where one is not (it lies on a face or beyond) or the table does not fit.
 static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
     const MGLevel& m = c.mg[0];
     GreenAxis ax[3];
@@ -527,7 +527,7 @@ static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
     if (doubles > (size_t)1 << 29) return false;   // 4 GiB
     double* pool = nullptr;
     int32_t* du = nullptr;
-    FOPIS_CUDA(cudaMallocAsync((void**)&pool, sizeof(double) * doubles, c.st));
+    if (cudaMallocAsync((void**)&pool, sizeof(double) * doubles, c.st) != cudaSuccess) { cudaGetLastError(); return false; }
     FOPIS_CUDA(cudaMallocAsync((void**)&du, sizeof(int32_t) * u.size(), c.st));
     FOPIS_CUDA(cudaMemcpyAsync(du, u.data(), sizeof(int32_t) * u.size(), cudaMemcpyHostToDevice, c.st));
     double* next = pool;
