@@ -1,14 +1,16 @@
 // multigrid.cu — the Poisson solve of RootGrid::solvePoisson
-// (src/Grid/RootGrid/RootGridField.cpp:41-103) as geometric multigrid.
+// (src/Grid/RootGrid/RootGridField.cpp:41-103) as FP64 iterative refinement.
 //
 // The reference sweeps plane-parity PSOR up to 1000 times per solve. Here the
 // FP64 outer loop computes r = f - A phi on the glue-layout node array
-// (f = rho0/eps0, A = 6 - sum of the six neighbours, dx = 1), and each
-// iteration solves A e = r approximately with one FP32 V-cycle (red-black
-// SOR smoothing with omega = 1.15, two sweeps before and one after the coarse
-// correction, full-weighting restriction, trilinear prolongation,
-// rediscretised coarse operators, single-CTA FP64 coarsest solve), then adds
-// e to phi in FP64. It stops when ||r||_2 <= tol ||f||_2.
+// (f = rho0/eps0, A = 6 - sum of the six neighbours, dx = 1), each iteration
+// solves A e = r in FP32 and adds e to phi in FP64, until
+// ||r||_2 <= tol ||f||_2. The correction is the fast diagonalisation of
+// direct.cu, or, on an axis of more than kDirectMax unknowns and for the EM
+// solver's start-up, one multigrid V-cycle (red-black SOR smoothing with omega
+// = 1.15, two sweeps before and one after the coarse correction,
+// full-weighting restriction, trilinear prolongation, rediscretised coarse
+// operators, single-CTA FP64 coarsest solve).
 //
 // Unknowns are the nodes the reference's PSOR updates: glue indices 1..n on a
 // periodic axis, 2..nx-1 on a Dirichlet/Neumann axis (Dirichlet and Neumann

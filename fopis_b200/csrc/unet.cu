@@ -21,11 +21,11 @@
 // computes 128 consecutive positions (M = 128) x COUT channels (N) in TMEM.
 // The 27 taps are grouped by (di, dj) into 9 stages; a stage stages the 130
 // positions of each input plane that the three dk taps read, plus the three
-// taps' weights, with cp.async into shared memory. The A operand of tap dk is
+// taps' weights, with bulk copies into shared memory. The A operand of tap dk is
 // the staged segment started dk rows later (K-major, rows 16 B apart), so no
 // im2col copy is made. Weight gradient: tcgen05 with both operands MN-major,
-// positions as K: A rows are (tap, input channel) built by 16-byte shifted
-// copies, B is the output gradient; partial sums leave TMEM through FP32
+// positions as K: A rows are (di, dj, input channel), read from one position
+// later for each dk, B is the output gradient; partial sums leave TMEM through FP32
 // atomics.
 #include "internal.cuh"
 #include "tc.cuh"

@@ -118,7 +118,7 @@ typedef struct fopis_params {
     int nspecies;                /* Environment::num_of_particle_types; order ambient -> photo */
     fopis_species species[FOPIS_MAX_SPECIES];
     double poisson_tol;          /* ||f - A phi||_2 <= tol ||f||_2 ; 0 -> 1e-8 */
-    int max_vcycles;             /* V-cycle cap per solve; 0 -> 100 */
+    int max_vcycles;             /* cap on corrections (V-cycles) per solve; 0 -> 100 */
     int guess_mode;              /* fopis_guess_mode */
     int sort_interval;           /* counting-sort period in steps; 0 -> 8 */
     int remove_interval;         /* removeInvalidParticles period (RootGrid.cpp:136-140); 0 -> 50 */
@@ -188,12 +188,12 @@ typedef enum fopis_field {
 
 typedef struct fopis_stats {
     int64_t timestep;            /* steps taken by this context */
-    int vcycles_last;            /* V-cycles of the last solve */
-    int vcycles_step;            /* V-cycles summed over the solves of the last step */
+    int vcycles_last;            /* corrections (V-cycles) of the last solve */
+    int vcycles_step;            /* corrections summed over the solves of the last step */
     int solves_step;             /* solves in the last step (2 with conductors) */
     int converged;               /* last solve reached the tolerance */
     double residual_last;        /* ||r||_2/||f||_2 of the last solve */
-    double residual_initial;     /* same, before the first V-cycle of the last solve */
+    double residual_initial;     /* same, before the first correction of the last solve */
     int64_t num_particles[FOPIS_MAX_SPECIES];   /* slots in use per species: the valid particles plus the
                                                    slots of particles removed since the last sort */
     int64_t capacity[FOPIS_MAX_SPECIES];
