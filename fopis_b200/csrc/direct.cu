@@ -308,7 +308,8 @@ template <bool BACK, int T>
 __global__ void __launch_bounds__(kThreads, 2) direct_rows_kernel(DirectShape S, DirectOuter O, float* X, double* phi) {
     extern __shared__ __align__(16) float sm[];
     constexpr int TS = T + 4;
-    constexpr int kBatch = 4;
+    constexpr int kBatch = T / kWarps < 4 ? T / kWarps : 4;
+    static_assert(T % (kBatch * kWarps) == 0, "whole batches of lines");
     const DirectAxis& x = S.ax[2];
     float* U = sm;
     float* V = U + 2 * x.hp * TS;
@@ -513,9 +514,12 @@ __global__ void __launch_bounds__(kThreads) direct_residual_kernel(DirectShape S
 size_t ring_smem(const DirectAxis& x) { return sizeof(float) * kStages * 2 * kRows * pass_modes(x.hp); }
 size_t tile_smem(const DirectAxis& x, int row) { return sizeof(float) * 4 * x.hp * row + ring_smem(x); }
 constexpr size_t kMostSmem = 224 * 1024;
-// Lines of a tile: 64 while such CTAs give every SM one and fit its shared memory.
+// Lines of a tile: 64 while such CTAs give every SM one and fit its shared memory,
+// else 32; 16 on axes (beyond 640 unknowns) of which 32 lines do not fit:
+// 213 KB on the longest, 1020 unknowns, with a quarter of the threads multiplying.
 int tile_lines(const DirectAxis& x, int lines, int pad) {
-    return lines >= 64 * 148 && tile_smem(x, 64 + pad) <= kMostSmem ? 64 : 32;
+    if (lines >= 64 * 148 && tile_smem(x, 64 + pad) <= kMostSmem) return 64;
+    return tile_smem(x, 32 + pad) <= kMostSmem ? 32 : 16;
 }
 
 // One axis' basis: folded index p (pairs, then self-mirrored ones) times mode
@@ -570,10 +574,10 @@ void build_axis(DirectAxis& x, int n, int per) {
 
 }  // namespace
 
-bool direct_fits(const int n[3]) { return n[0] <= kDirectMax && n[1] <= kDirectMax && n[2] <= kDirectMax; }
+bool direct_first(const int n[3]) { return n[0] <= kDirectMax && n[1] <= kDirectMax && n[2] <= kDirectMax; }
 
-int direct_blocks(const DirectShape& S) {
-    const long long tiles = (long long)((S.n2 + 31) / 32) * ((S.n1 + 7) / 8) * ((S.n0 + kResA - 1) / kResA);
+int direct_blocks(const int n[3]) {
+    const long long tiles = (long long)((n[2] + 31) / 32) * ((n[1] + 7) / 8) * ((n[0] + kResA - 1) / kResA);
     return (int)std::min<long long>(tiles, 148 * 8);
 }
 
@@ -595,18 +599,16 @@ void launch_cols(const DirectShape& S, float* X, bool pdl, cudaStream_t st) {
     const DirectAxis& x = S.ax[MODE == 1 ? 0 : 1];
     const int lines = MODE == 1 ? S.n1 * S.n2 : S.n0 * S.n2, T = tile_lines(x, lines, 0);
     const dim3 grid((lines + T - 1) / T);
-    if (T == 64) launch_k(pdl, direct_cols_kernel<MODE, 64>, grid, dim3(kThreads), tile_smem(x, T), st, S, X);
-    else launch_k(pdl, direct_cols_kernel<MODE, 32>, grid, dim3(kThreads), tile_smem(x, T), st, S, X);
+    auto* kernel = T == 64 ? direct_cols_kernel<MODE, 64> : (T == 32 ? direct_cols_kernel<MODE, 32> : direct_cols_kernel<MODE, 16>);
+    launch_k(pdl, kernel, grid, dim3(kThreads), tile_smem(x, T), st, S, X);
 }
 template <bool BACK>
 void launch_rows(const DirectShape& S, const DirectOuter& O, float* X, double* phi, bool pdl, cudaStream_t st) {
     const DirectAxis& x = S.ax[2];
     const int lines = S.n0 * S.n1, T = tile_lines(x, lines, 4);
     const dim3 grid((lines + T - 1) / T);
-    if (T == 64)
-        launch_k(pdl, direct_rows_kernel<BACK, 64>, grid, dim3(kThreads), tile_smem(x, T + 4), st, S, O, X, phi);
-    else
-        launch_k(pdl, direct_rows_kernel<BACK, 32>, grid, dim3(kThreads), tile_smem(x, T + 4), st, S, O, X, phi);
+    auto* kernel = T == 64 ? direct_rows_kernel<BACK, 64> : (T == 32 ? direct_rows_kernel<BACK, 32> : direct_rows_kernel<BACK, 16>);
+    launch_k(pdl, kernel, grid, dim3(kThreads), tile_smem(x, T + 4), st, S, O, X, phi);
 }
 }  // namespace
 
@@ -616,6 +618,7 @@ void direct_setup(DirectShape& S, const int n[3], const int per[3]) {
     // the attribute belongs to the function, which contexts of other sizes share
     allow_tile<64>();
     allow_tile<32>();
+    allow_tile<16>();
 }
 
 void direct_free(DirectShape& S) {
@@ -628,7 +631,8 @@ void direct_free(DirectShape& S) {
 // X = f - A phi and the decision of `step`.
 int direct_residual(const DirectShape& S, const DirectOuter& O, const double* rho0, const double* phi, float* X,
                     double* partial, const DirectStep& step, bool pdl, cudaStream_t st) {
-    launch_k(pdl, direct_residual_kernel, dim3(direct_blocks(S)), dim3(kThreads), 0, st, S, O, rho0, phi, X, partial, step);
+    const int n[3] = {S.n0, S.n1, S.n2};
+    launch_k(pdl, direct_residual_kernel, dim3(direct_blocks(n)), dim3(kThreads), 0, st, S, O, rho0, phi, X, partial, step);
     return 1;
 }
 

@@ -29,8 +29,8 @@ struct DirectStep {
     cudaGraphConditionalHandle loop;
 };
 
-bool direct_fits(const int n[3]);
-int direct_blocks(const DirectShape& S);
+bool direct_first(const int n[3]);   // corrections by this from the start, and not only where V-cycles fail
+int direct_blocks(const int n[3]);
 void direct_setup(DirectShape& S, const int n[3], const int per[3]);
 void direct_free(DirectShape& S);
 int direct_residual(const DirectShape& S, const DirectOuter& O, const double* rho0, const double* phi, float* X,

@@ -10,7 +10,11 @@
 // solver's start-up, one multigrid V-cycle (red-black SOR smoothing with omega
 // = 1.15, two sweeps before and one after the coarse correction,
 // full-weighting restriction, trilinear prolongation, rediscretised coarse
-// operators, single-CTA FP64 coarsest solve).
+// operators, single-CTA FP64 coarsest solve). Halving an even count between held
+// faces puts the coarse far face one fine cell too far out, and a few such levels
+// over-correct: V-cycles reach 1e-8 only slowly (42^3 nodes) or diverge (50^3 and
+// many larger ones). A solve whose V-cycles fail hands the context over to the
+// direct corrections, which take any axis length (mg_to_direct).
 //
 // Unknowns are the nodes the reference's PSOR updates: glue indices 1..n on a
 // periodic axis, 2..nx-1 on a Dirichlet/Neumann axis (Dirichlet and Neumann
@@ -1403,12 +1407,13 @@ void mg_setup(Ctx& c) {
     // V-cycles: from a potential that differs in its last digits a few particles in
     // 1e8 move to the other side of a cell face within some steps, and a move that
     // changes its cell puts v^2 of its charge on other edges than one that does not.
-    c.direct = !c.em.on && direct_fits(c.mg[0].n);
+    // (Where they fail, the direct corrections take over there too.)
+    c.direct = !c.em.on && direct_first(c.mg[0].n);
     if (c.direct) {
         MGLevel& l = c.mg[0];
         FOPIS_CUDA(cudaMalloc(&l.f, sizeof(float) * l.size()));
         direct_setup(c.dir, l.n, l.per);
-        c.red_blocks = std::max(kRedBlocks, direct_blocks(c.dir));
+        c.red_blocks = std::max(kRedBlocks, direct_blocks(l.n));
         FOPIS_CUDA(cudaMalloc(&c.red_partials, sizeof(double) * 3 * c.red_blocks));
         return;
     }
@@ -1448,17 +1453,52 @@ void mg_setup(Ctx& c) {
     FOPIS_CUDA(cudaMalloc(&c.red_partials, sizeof(double) * 2 * 148 * 8));
 }
 
-void mg_free(Ctx& c) {
+static void drop_graphs(Ctx& c) {
     if (c.mg_exec) { cudaGraphExecDestroy(c.mg_exec); c.mg_exec = nullptr; }
     if (c.mg_graph) { cudaGraphDestroy(c.mg_graph); c.mg_graph = nullptr; }
     if (c.solve_exec) { cudaGraphExecDestroy(c.solve_exec); c.solve_exec = nullptr; }
     if (c.solve_graph) { cudaGraphDestroy(c.solve_graph); c.solve_graph = nullptr; }
     if (c.body_st) { cudaStreamDestroy(c.body_st); c.body_st = nullptr; }
     c.solve_state = 0;
+}
+
+void mg_free(Ctx& c) {
+    drop_graphs(c);
     for (auto& l : c.mg) { cudaFree(l.u); cudaFree(l.f); cudaFree(l.r); }
     c.mg.clear();
     direct_free(c.dir);
     if (c.red_partials) { cudaFree(c.red_partials); c.red_partials = nullptr; }
+}
+
+// Gives a context of V-cycles the direct corrections for the rest of its life;
+// false, with the V-cycles kept, where their tables cannot be allocated.
+static bool mg_to_direct(Ctx& c) {
+    FOPIS_CUDA(cudaStreamSynchronize(c.st));
+    double* partials = nullptr;
+    const int blocks = std::max(kRedBlocks, direct_blocks(c.mg[0].n));
+    try {
+        direct_setup(c.dir, c.mg[0].n, c.mg[0].per);
+        FOPIS_CUDA(cudaMalloc(&partials, sizeof(double) * 3 * blocks));
+        FOPIS_CUDA(cudaDeviceSynchronize());   // the tables are there before c.st reads them
+    } catch (const CudaError& e) {
+        cudaGetLastError();
+        direct_free(c.dir);
+        if (e.code != cudaErrorMemoryAllocation) throw;
+        return false;
+    }
+    drop_graphs(c);
+    for (size_t l = 0; l < c.mg.size(); ++l) {   // the finest right-hand side stays
+        MGLevel& m = c.mg[l];
+        cudaFree(m.u);
+        cudaFree(m.r);
+        m.u = m.r = nullptr;
+        if (l > 0) { cudaFree(m.f); m.f = nullptr; }
+    }
+    cudaFree(c.red_partials);
+    c.red_partials = partials;
+    c.red_blocks = blocks;
+    c.direct = true;
+    return true;
 }
 
 // The FP64 side of the direct correction's kernels.
@@ -1545,6 +1585,8 @@ __global__ void solve_prep_kernel(DevScalars* sc, double M, int allper) {
     const double fn = sqrt(fmax(0.0, fsq - (allper ? fsum * fsum / M : 0.0)));
     sc->red[5] = fn > 0.0 ? fn : 1.0;
 }
+// V-cycles that diverge are given up at this many times the first residual.
+constexpr double kDiverged = 1e3;
 // Loop condition: residual above tolerance, cap not reached, residual finite.
 __global__ void solve_init_kernel(DevScalars* sc, cudaGraphConditionalHandle h) {
     pdl_entry();
@@ -1568,7 +1610,7 @@ __global__ void solve_decide_kernel(const double* partial, int nparts, DevScalar
         const double n = sc->red[8] + 1.0;
         sc->red[8] = n;
         const double res = sqrt(v);
-        const bool go = isfinite(res) && res > sc->red[6] * sc->red[5] && n < sc->red[7];
+        const bool go = isfinite(res) && res > sc->red[6] * sc->red[5] && n < sc->red[7] && res <= kDiverged * sc->red[9];
         cudaGraphSetConditional(h, go ? 1u : 0u);
     }
 }
@@ -1721,13 +1763,14 @@ void mg_solve_host_loop(Ctx& c, double tol, int max_cycles, double* res_out, dou
     }
     c.first_res = res / fnorm;
     int cycles = 0;
+    const double most = c.direct ? HUGE_VAL : kDiverged * res;
     while (res > tol * fnorm && cycles < max_cycles) {
         FOPIS_CUDA(cudaGraphLaunch(c.mg_exec, c.st));
         c.launches += c.cycle_launches;
         FOPIS_CUDA(cudaStreamSynchronize(c.st));
         res = std::sqrt(c.h_sc->red[2]);
         ++cycles;
-        if (!std::isfinite(res)) break;
+        if (!std::isfinite(res) || res > most) break;
     }
     if (allper) {
         ++c.launches;
@@ -1768,22 +1811,37 @@ void mg_prepare(Ctx& c) {
     }
 }
 
-int mg_solve(Ctx& c, double tol, int max_cycles) {
+static void run_solve(Ctx& c, double tol, int max_cycles, double* res, double* fnorm, int* cycles) {
     mg_prepare(c);
-    double res = 0.0, fnorm = 1.0;
-    int cycles = 0;
     if (c.solve_state == 1) {
         c.h_sc->red[6] = tol;
         c.h_sc->red[7] = (double)max_cycles;
         FOPIS_CUDA(cudaGraphLaunch(c.solve_exec, c.st));
         FOPIS_CUDA(cudaStreamSynchronize(c.st));
-        fnorm = c.h_sc->red[5];
-        res = std::sqrt(c.h_sc->red[2]);
-        cycles = (int)c.h_sc->red[8];
-        c.first_res = c.h_sc->red[9] / fnorm;
-        c.launches += c.solve_pre_launches + (int64_t)cycles * c.cycle_launches + c.solve_post_launches;
+        *fnorm = c.h_sc->red[5];
+        *res = std::sqrt(c.h_sc->red[2]);
+        *cycles = (int)c.h_sc->red[8];
+        c.first_res = c.h_sc->red[9] / *fnorm;
+        c.launches += c.solve_pre_launches + (int64_t)*cycles * c.cycle_launches + c.solve_post_launches;
     } else {
-        mg_solve_host_loop(c, tol, max_cycles, &res, &fnorm, &cycles);
+        mg_solve_host_loop(c, tol, max_cycles, res, fnorm, cycles);
+    }
+}
+
+int mg_solve(Ctx& c, double tol, int max_cycles) {
+    double res = 0.0, fnorm = 1.0;
+    int cycles = 0;
+    run_solve(c, tol, max_cycles, &res, &fnorm, &cycles);
+    // V-cycles that work halve the residual at the least (they end at a low cap with
+    // the tolerance unmet, no more); where they do not, start again from zero with the
+    // direct corrections.
+    const double first = c.first_res * fnorm;
+    if (!c.direct && cycles > 0 && std::isfinite(first) && !(res <= tol * fnorm) &&
+        !(res <= first * std::pow(0.5, cycles)) && mg_to_direct(c)) {
+        const int before = cycles;
+        FOPIS_CUDA(cudaMemsetAsync(c.phi, 0, sizeof(double) * c.N, c.st));
+        run_solve(c, tol, max_cycles, &res, &fnorm, &cycles);
+        cycles += before;
     }
     if (!c.direct) {   // the reference's pointwise measure on the state the solve reached (faces still held)
         const Outer O = make_outer(c);
