@@ -413,8 +413,10 @@ void object_upload(Ctx& c, ObjectDev& o, const fopis_object_desc* d, int id) {
         cmap[((size_t)i * c.cy + j) * c.cz + k] = (uint8_t)(id + 1);
         h.cells[((size_t)i * (c.ny + 1) + j) * (c.nz + 1) + k] = 1;
     }
-    FOPIS_CUDA(cudaMemcpy(c.node_cmat, ncm.data(), sizeof(int32_t) * c.N, cudaMemcpyHostToDevice));
-    FOPIS_CUDA(cudaMemcpy(c.cellmap, cmap.data(), c.N, cudaMemcpyHostToDevice));
+    // in the order of c.st, which a plain copy is not ordered with: it may return before
+    // its last piece is on the device, and the marks are read from the map only here
+    copy_to_device(c, c.node_cmat, ncm.data(), sizeof(int32_t) * c.N);
+    copy_to_device(c, c.cellmap, cmap.data(), c.N);
     mark_brick_bodies(c);
     FOPIS_CUDA(cudaMalloc(&o.nodes, sizeof(int32_t) * o.n));
     FOPIS_CUDA(cudaMemcpy(o.nodes, lin.data(), sizeof(int32_t) * o.n, cudaMemcpyHostToDevice));
