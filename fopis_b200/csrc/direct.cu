@@ -384,9 +384,9 @@ __device__ __forceinline__ int wrap_node(int idx, int per, int nref) {
     return idx;
 }
 
-// A thread's share of the residual's sums.
+// A thread's share of the residual's sums (rsum where every axis is periodic).
 struct ResidualSums {
-    double f2 = 0.0, r2 = 0.0, worst = 0.0;
+    double f2 = 0.0, r2 = 0.0, rsum = 0.0, worst = 0.0;
 };
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -398,17 +398,18 @@ __device__ __forceinline__ double warp_max(double v) {
     return v;
 }
 
-// Block totals of the three sums in thread 0 (fixed order).
-__device__ ResidualSums block_sums(ResidualSums s) {
-    __shared__ double red[3][kWarps];
+// Block totals of the sums in thread 0 (fixed order).
+__device__ ResidualSums block_sums(ResidualSums s, bool allper) {
+    __shared__ double red[4][kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     s.f2 = warp_sum(s.f2); s.r2 = warp_sum(s.r2); s.worst = warp_max(s.worst);
+    if (allper) s.rsum = warp_sum(s.rsum);
     __syncthreads();
-    if (lane == 0) { red[0][warp] = s.f2; red[1][warp] = s.r2; red[2][warp] = s.worst; }
+    if (lane == 0) { red[0][warp] = s.f2; red[1][warp] = s.r2; red[2][warp] = s.worst; red[3][warp] = s.rsum; }
     __syncthreads();
     if (threadIdx.x == 0)
         for (int w = 1; w < kWarps; ++w) {
-            s.f2 += red[0][w]; s.r2 += red[1][w];
+            s.f2 += red[0][w]; s.r2 += red[1][w]; s.rsum += red[3][w];
             s.worst = red[2][w] > s.worst ? red[2][w] : s.worst;
         }
     return s;
@@ -416,15 +417,21 @@ __device__ ResidualSums block_sums(ResidualSums s) {
 
 // The end of a residual: the refinement's scalars, and with DIRECT_LOOP whether
 // the graph's loop takes another correction (tolerance not met, cap not
-// reached, residual finite).
-__device__ void decide(const DirectStep& d, double f2, double r2, double worst) {
+// reached, residual finite). In an all-periodic box the mean of f, subtracted as a
+// rounded number, leaves a constant of a rounding or so in f and in every r, which
+// no phi can lower: it is taken out of both norms (M: the unknowns' number). And
+// charge that differs from its mean by less than a rounding of the mean over the
+// tolerance (1e-8 of it at 1e-8) is solved to that rounding instead: fm carries it.
+__device__ void decide(const DirectStep& d, const ResidualSums& t, double M, double fm) {
     double* red = d.sc->red;
+    const double constant = t.rsum * (t.rsum / M);
+    const double r2 = t.r2 >= constant ? t.r2 - constant : (isfinite(t.r2) ? 0.0 : t.r2), worst = t.worst;
     const double res = sqrt(r2);
     if (d.mode & DIRECT_START) {
-        const double fn = sqrt(f2);
-        red[5] = fn > 0.0 ? fn : 1.0;
         red[6] = d.host->red[6];
         red[7] = d.host->red[7];
+        double fn = fmax(sqrt(fmax(t.f2 - constant, 0.0)), 0x1p-53 * fabs(fm) * sqrt(M) / red[6]);
+        red[5] = fn > 0.0 ? fn : 1.0;
         red[8] = 0.0;
         red[9] = res;
     } else {
@@ -486,13 +493,14 @@ __global__ void __launch_bounds__(kThreads) direct_residual_kernel(DirectShape S
             X[((long long)a * S.n1 + b) * S.n2 + c] = (float)r[e];
             sums.f2 += src[e] * src[e];
             sums.r2 += r[e] * r[e];
+            if (O.allper) sums.rsum += r[e];
             if (src[e] != 0.0 && fabs(r[e]) > sums.worst * fabs(src[e])) sums.worst = fmax(sums.worst, fabs(r[e] / src[e]));
         }
     }
-    sums = block_sums(sums);
+    sums = block_sums(sums, O.allper);
     if (threadIdx.x == 0) {
-        double* p = partial + 3 * (long long)blockIdx.x;
-        p[0] = sums.f2; p[1] = sums.r2; p[2] = sums.worst;
+        double* p = partial + kDirectPartials * (long long)blockIdx.x;
+        p[0] = sums.f2; p[1] = sums.r2; p[2] = sums.worst; p[3] = sums.rsum;
         __threadfence();
         s_last = atomicInc(&step.sc->ticket, gridDim.x - 1) == gridDim.x - 1;
     }
@@ -501,14 +509,14 @@ __global__ void __launch_bounds__(kThreads) direct_residual_kernel(DirectShape S
     __threadfence();
     ResidualSums t;
     for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
-        const volatile double* p = partial + 3 * (long long)b;
-        t.f2 += p[0]; t.r2 += p[1];
+        const volatile double* p = partial + kDirectPartials * (long long)b;
+        t.f2 += p[0]; t.r2 += p[1]; t.rsum += p[3];
         const double w = p[2];
         t.worst = w > t.worst ? w : t.worst;
     }
-    t = block_sums(t);
+    t = block_sums(t, O.allper);
     if (threadIdx.x != 0) return;
-    decide(step, t.f2, t.r2, t.worst);
+    decide(step, t, (double)S.n0 * S.n1 * S.n2, fm);
 }
 
 size_t ring_smem(const DirectAxis& x) { return sizeof(float) * kStages * 2 * kRows * pass_modes(x.hp); }

@@ -29,6 +29,8 @@ struct DirectStep {
     cudaGraphConditionalHandle loop;
 };
 
+constexpr int kDirectPartials = 4;   // doubles per block of direct_residual's `partial`
+
 bool direct_first(const int n[3]);   // corrections by this from the start, and not only where V-cycles fail
 int direct_blocks(const int n[3]);
 void direct_setup(DirectShape& S, const int n[3], const int per[3]);

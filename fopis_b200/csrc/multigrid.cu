@@ -1414,7 +1414,7 @@ void mg_setup(Ctx& c) {
         FOPIS_CUDA(cudaMalloc(&l.f, sizeof(float) * l.size()));
         direct_setup(c.dir, l.n, l.per);
         c.red_blocks = std::max(kRedBlocks, direct_blocks(l.n));
-        FOPIS_CUDA(cudaMalloc(&c.red_partials, sizeof(double) * 3 * c.red_blocks));
+        FOPIS_CUDA(cudaMalloc(&c.red_partials, sizeof(double) * kDirectPartials * c.red_blocks));
         return;
     }
     for (auto& l : c.mg) {
@@ -1478,7 +1478,7 @@ static bool mg_to_direct(Ctx& c) {
     const int blocks = std::max(kRedBlocks, direct_blocks(c.mg[0].n));
     try {
         direct_setup(c.dir, c.mg[0].n, c.mg[0].per);
-        FOPIS_CUDA(cudaMalloc(&partials, sizeof(double) * 3 * blocks));
+        FOPIS_CUDA(cudaMalloc(&partials, sizeof(double) * kDirectPartials * blocks));
         FOPIS_CUDA(cudaDeviceSynchronize());   // the tables are there before c.st reads them
     } catch (const CudaError& e) {
         cudaGetLastError();
@@ -1735,6 +1735,8 @@ void mg_solve_host_loop(Ctx& c, double tol, int max_cycles, double* res_out, dou
     const long long M = (long long)O.n0 * O.n1 * O.n2;
     double fnorm = 1.0, res = 0.0;
     if (c.direct) {
+        c.h_sc->red[6] = tol;
+        c.h_sc->red[7] = (double)max_cycles;
         direct_begin(c, O, DirectStep{c.d_sc, c.h_sc, DIRECT_START, 0});
         FOPIS_CUDA(cudaStreamSynchronize(c.st));
         fnorm = c.h_sc->red[5];

@@ -89,3 +89,30 @@ def test_em_solves_where_v_cycles_fail(gpu_available, n, boundary, boxes):
         st = g.stats()
         assert st.converged and st.solves_step == 1 and 1 <= st.vcycles_step <= 3
     g.close()
+
+
+@pytest.mark.parametrize("nxyz", [(16, 16, 16), (17, 18, 19), (96, 80, 100)])
+def test_near_uniform_periodic_charge(gpu_available, nxyz):
+    """Charge that is its mean, or differs from it by little more than roundings: solved to the tolerance, or to a
+    rounding of the mean where that is more, from zero and from the last potential."""
+    dx, dt = plasma_units()
+    sp = [SpeciesInfo("Electron", "ambient", 1.0, -1.0, 1e7, 1.0, 1)]
+    p, norm = make_params(nxyz, "PPPPPP", dx, dt, sp)
+    g = RootGrid(config.SimConfig(params=p, norm=norm, species=sp))
+    tol, inner = 1e-8, (slice(1, -1),) * 3
+    rng = np.random.default_rng(4)
+    for value in (1.0, 0.3, 1e6, 123456.789, -7.7e3, 3e-12, 1.0 / 3.0):
+        for noise in (0.0, 1e-15, 1e-12, 1e-10, 1e-8):
+            rho = np.pad(value * (1.0 + noise * rng.standard_normal(nxyz)), 1, mode="wrap")
+            g.set_guess_mode(_abi.GUESS_ZERO if rng.random() < 0.5 else _abi.GUESS_WARM)
+            g.set_field(_abi.FIELD_RHO0, rho)
+            assert g.solvePoisson() == 0, (value, noise, g.stats().residual_last)
+            phi = g.getPhi()
+            f = rho[inner] / p.eps0
+            r = f - f.mean() - 6.0 * phi[inner]
+            for a in range(3):
+                r += np.roll(phi[inner], 1, axis=a) + np.roll(phi[inner], -1, axis=a)
+            # a rounding of the mean, as much again for the storing of phi (which the mean's removal rounds anew)
+            most = tol * np.linalg.norm(f - f.mean()) + (2.0 ** -53 * abs(f.mean()) + 24 * 2.0 ** -53 * np.abs(phi).max()) * np.sqrt(f.size)
+            assert np.linalg.norm(r - r.mean()) <= most
+    g.close()
