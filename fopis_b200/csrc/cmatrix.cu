@@ -4,8 +4,8 @@
 // Capacity matrix (RootGrid::initializeObjectsCmatrix, RootGridObject.cpp:77-148):
 // column c of B holds phi at every surface node for rho = 1 at surface node c:
 // values of the grid's Green's function, from one table over node differences
-// and sums (one multigrid or direct solve per column where a surface node is
-// not an unknown of the solve); C = B^-1 by blocked in-place Gauss-Jordan
+// and sums (one solve per column where the table takes more than 4 GiB or cannot
+// be allocated); C = B^-1 by blocked in-place Gauss-Jordan
 // elimination in FP64 on the device (B is symmetric positive definite, so no
 // pivoting). Per step (Spacecraft::redistributeChargeForPerfectConductor,
 // Spacecraft.cpp:708-758): V = (sum_ij C_ij phi_j + Q) / sum_ij C_ij, or the
@@ -380,6 +380,21 @@ struct HostObj {
     }
 };
 
+// A buffer of the context's stream, given back in its order.
+template <typename T>
+struct StreamBuffer {
+    Ctx& c;
+    T* p = nullptr;
+    explicit StreamBuffer(Ctx& x) : c(x) {}
+    ~StreamBuffer() { if (p) cudaFreeAsync(p, c.st); }
+    bool alloc(size_t n) {
+        if (cudaMallocAsync((void**)&p, sizeof(T) * n, c.st) == cudaSuccess) return true;
+        cudaGetLastError();
+        p = nullptr;
+        return false;
+    }
+};
+
 int grid1(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + kT - 1) / kT, 148LL * 16)); }
 
 }  // namespace
@@ -502,8 +517,9 @@ static void finish_C(Ctx& c, ObjectDev& o) {
     }
 }
 
-// B of an object whose surface nodes are all unknowns of the Poisson solve;
-// false where one is not (it lies on a face or beyond) or the table does not fit.
+// B of an object from the table; false where the table does not fit. A surface
+// node that is no unknown of the Poisson solve (it lies on a face or beyond) takes
+// no charge: its column of B is zero.
 static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
     const MGLevel& m = c.mg[0];
     GreenAxis ax[3];
@@ -513,7 +529,8 @@ static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
         int lo = 1 << 30, hi = 0;
         for (int t = 0; t < o.n; ++t) {
             const int q = o.nodes_ijk[3 * (size_t)t + d] - first + 1;
-            if (q < 1 || q > m.n[d]) return false;
+            if (q < 1 || q > m.n[d])
+                throw ApiError{FOPIS_ERR_DEVICE, "capacity matrix B is not positive definite: a surface node is on a face"};
             u[(size_t)d * o.n + t] = q;
             lo = std::min(lo, q);
             hi = std::max(hi, q);
@@ -527,12 +544,11 @@ static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
     for (const auto& x : ax) tables += (size_t)x.n * (x.count + 1);
     const size_t doubles = tables + first + second + third;
     if (doubles > (size_t)1 << 29) return false;   // 4 GiB
-    double* pool = nullptr;
-    int32_t* du = nullptr;
-    if (cudaMallocAsync((void**)&pool, sizeof(double) * doubles, c.st) != cudaSuccess) { cudaGetLastError(); return false; }
-    FOPIS_CUDA(cudaMallocAsync((void**)&du, sizeof(int32_t) * u.size(), c.st));
-    FOPIS_CUDA(cudaMemcpyAsync(du, u.data(), sizeof(int32_t) * u.size(), cudaMemcpyHostToDevice, c.st));
-    double* next = pool;
+    StreamBuffer<double> pool(c);
+    StreamBuffer<int32_t> du(c);
+    if (!pool.alloc(doubles) || !du.alloc(u.size())) return false;
+    FOPIS_CUDA(cudaMemcpyAsync(du.p, u.data(), sizeof(int32_t) * u.size(), cudaMemcpyHostToDevice, c.st));
+    double* next = pool.p;
     for (auto& x : ax) {
         x.cosines = next;
         x.lambda = next + (size_t)x.n * x.count;
@@ -550,10 +566,8 @@ static bool green_matrix(Ctx& c, const ObjectDev& o, double* B) {
     };
     contract(ax[1], R1, ax[2].count, ax[0].n, R2);
     contract(ax[0], R2, ax[1].count * ax[2].count, 1, T);
-    green_matrix_kernel<<<grid1((long long)o.n * o.n), kT, 0, c.st>>>(ax[0], ax[1], ax[2], T, du, o.n, 1.0 / c.p.eps0, B);
+    green_matrix_kernel<<<grid1((long long)o.n * o.n), kT, 0, c.st>>>(ax[0], ax[1], ax[2], T, du.p, o.n, 1.0 / c.p.eps0, B);
     FOPIS_LAUNCH_CHECK();
-    FOPIS_CUDA(cudaFreeAsync(pool, c.st));
-    FOPIS_CUDA(cudaFreeAsync(du, c.st));
     FOPIS_CUDA(cudaStreamSynchronize(c.st));   // the node list is a local
     return true;
 }
@@ -586,22 +600,20 @@ void cmatrix_build(Ctx& c, int id) {
     FOPIS_CUDA(cudaMemsetAsync(c.rho0, 0, sizeof(double) * c.N, c.st));
     if (!green_matrix(c, o, B)) solved_matrix(c, o, B);
     FOPIS_CUDA(cudaMemsetAsync(c.phi, 0, sizeof(double) * c.N, c.st));
-    double* row = nullptr;
-    unsigned* bad = nullptr;
-    FOPIS_CUDA(cudaMallocAsync((void**)&row, sizeof(double) * 2 * kGj * n, c.st));
-    FOPIS_CUDA(cudaMallocAsync((void**)&bad, sizeof(unsigned), c.st));
-    FOPIS_CUDA(cudaMemsetAsync(bad, 0, sizeof(unsigned), c.st));
+    StreamBuffer<double> panels(c);
+    StreamBuffer<unsigned> bad(c);
+    if (!panels.alloc((size_t)2 * kGj * n) || !bad.alloc(1)) FOPIS_CUDA(cudaErrorMemoryAllocation);
+    double *row = panels.p, *col = row + (size_t)kGj * n;
+    FOPIS_CUDA(cudaMemsetAsync(bad.p, 0, sizeof(unsigned), c.st));
     const int tiles = (n + kGjTile - 1) / kGjTile;
     for (int k = 0; k < n; k += kGj) {
         c.launches += 2;
-        gj_panel_kernel<<<(n + 255) / 256, 256, 0, c.st>>>(B, n, k, row, row + (size_t)kGj * n, bad);
-        gj_update_kernel<<<dim3(tiles, tiles), 256, 0, c.st>>>(B, n, k, row, row + (size_t)kGj * n);
+        gj_panel_kernel<<<(n + 255) / 256, 256, 0, c.st>>>(B, n, k, row, col, bad.p);
+        gj_update_kernel<<<dim3(tiles, tiles), 256, 0, c.st>>>(B, n, k, row, col);
     }
     FOPIS_LAUNCH_CHECK();
     unsigned hbad = 0;
-    FOPIS_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, c.st));
-    FOPIS_CUDA(cudaFreeAsync(row, c.st));
-    FOPIS_CUDA(cudaFreeAsync(bad, c.st));
+    FOPIS_CUDA(cudaMemcpyAsync(&hbad, bad.p, sizeof(unsigned), cudaMemcpyDeviceToHost, c.st));
     FOPIS_CUDA(cudaStreamSynchronize(c.st));
     if (hbad) throw ApiError{FOPIS_ERR_DEVICE, "capacity matrix B is not positive definite"};
     finish_C(c, o);

@@ -1,8 +1,9 @@
 """The capacity matrix from the Green's function table and the blocked inversion
 against numpy in FP64: held, periodic and mixed boxes, bodies off the centre and
 beside a face, fewer nodes than one 32-pivot step and counts that leave a
-remainder of it. A body on a face has no positive definite matrix and is still
-refused."""
+remainder of it. A body on a face has no positive definite matrix and is
+refused before any solve. Two parts so far apart that the table takes more than
+its 4 GiB go through one solve per node."""
 import numpy as np
 import pytest
 
@@ -12,11 +13,11 @@ from fopis_b200.config import SpeciesInfo, make_params, plasma_units
 pytestmark = pytest.mark.gpu
 
 
-def grid(nxyz, boundary, box):
+def grid(nxyz, boundary, *boxes):
     dx, dt = plasma_units()
     sp = [SpeciesInfo("Electron", "ambient", 1.0, -1.0, 1e7, 1.0, 1)]
     p, norm = make_params(nxyz, boundary, dx, dt, sp)
-    obj = config.objects_from_boxes([box], nxyz)
+    obj = config.objects_from_boxes(list(boxes), nxyz)
     return RootGrid(config.SimConfig(params=p, norm=norm, species=sp, objects=[obj])), p, obj
 
 
@@ -59,5 +60,36 @@ def test_body_on_a_face_is_refused(gpu_available):
     g, _, _ = grid((12, 12, 12), "DDDDDD", ((-6, -1, -1), (-3, 1, 1)))
     with pytest.raises(FopisError) as e:
         g.initializeObjectsCmatrix(0)
-    assert e.value.code in (_abi.ERR_DEVICE, _abi.ERR_NOT_CONVERGED)
+    assert e.value.code == _abi.ERR_DEVICE
+    assert g.stats().vcycles_step == 0
     g.close()
+
+
+def test_far_apart_parts_are_solved_node_by_node(gpu_available):
+    nxyz = (301, 300, 301)
+    g, p, obj = grid(nxyz, "DDDDDD", ((-146, -145, -144), (-145, -144, -143)), ((144, 143, 145), (145, 144, 146)))
+    nodes = np.asarray(obj.nodes, np.int64)
+    counts = [3 * int(np.ptp(nodes[:, a])) + 2 for a in range(3)]
+    assert np.prod(counts, dtype=np.int64) > 1 << 29   # doubles: the table does not fit
+    g.initializeObjectsCmatrix(0)
+    assert g.stats().vcycles_last >= 1                 # solved
+    C = g.get_cmatrix(0)
+    g.close()
+    # phi at every node for a unit charge at one: sines of each axis, one charge at a time
+    S, lam = [], []
+    for a in range(3):
+        n = nxyz[a] - 2
+        k = np.arange(1, n + 1)
+        S.append(np.sqrt(2.0 / (n + 1)) * np.sin(np.pi * np.outer(nodes[:, a] - 1, k) / (n + 1)))
+        lam.append(2.0 - 2.0 * np.cos(np.pi * k / (n + 1)))
+    inv = 1.0 / (lam[0][:, None, None] + lam[1][None, :, None] + lam[2][None, None, :])
+    B = np.empty((len(nodes), len(nodes)))
+    for j in range(len(nodes)):
+        t = (inv @ (S[2] * S[2][j]).T)                          # [k][l][i]
+        t = np.einsum("kli,il->ki", t, S[1] * S[1][j])
+        B[:, j] = np.einsum("ki,ik->i", t, S[0] * S[0][j])
+    B /= p.eps0
+    ref = np.linalg.inv(B)
+    # the solves go to ||r|| <= 1e-10 ||f||, phi off by at most 1e-10 / lambda_min of a unit charge
+    off = 1e-10 / min(l.min() for l in lam) / p.eps0 * len(B)
+    assert np.linalg.norm(C - ref, 2) <= 2.0 * np.linalg.norm(ref, 2) ** 2 * off
