@@ -95,6 +95,14 @@ struct Ring {
     ~Ring() { end(); }
 };
 
+// Waits for the copies between the device and the slots when a copy ends early, by
+// an error: the next one, another context's perhaps, fills the slots anew.
+struct Drain {
+    cudaStream_t st;
+    bool staged = false;
+    ~Drain() { if (staged) cudaStreamSynchronize(st); }
+};
+
 // Takes the ring and cuts the segments into chunks; false when the copy should
 // not be staged.
 bool begin(Ctx& c, const CopySegment* s, int n, Ring& r, std::unique_lock<std::mutex>& lock) {
@@ -137,7 +145,8 @@ void hostcopy_close(Ctx& c) {
 
 // Device to host in stream order; the memory is filled when it returns.
 void copy_to_host(Ctx& c, const CopySegment* s, int n) {
-    std::unique_lock<std::mutex> lock;   // released after the threads are joined
+    std::unique_lock<std::mutex> lock;   // released after the threads are joined and the slots at rest
+    Drain drain{c.st};
     Ring r;
     if (!begin(c, s, n, r, lock) || !r.start(true)) {
         for (int q = 0; q < n; ++q)
@@ -145,6 +154,7 @@ void copy_to_host(Ctx& c, const CopySegment* s, int n) {
         FOPIS_CUDA(cudaStreamSynchronize(c.st));
         return;
     }
+    drain.staged = true;
     const int total = (int)r.chunks.size();
     for (int issued = 0, landed = 0; landed < total;) {
         if (issued < total && issued - landed < kSlots &&
@@ -161,12 +171,14 @@ void copy_to_host(Ctx& c, const CopySegment* s, int n) {
         }
     }
     for (int i = 0; i < total; ++i) r.wait_done(i);
+    drain.staged = false;
 }
 
 // Host to device in stream order; the memory has been read when it returns,
 // without wait only once the stream has passed.
 void copy_to_device(Ctx& c, const CopySegment* s, int n, bool wait) {
     std::unique_lock<std::mutex> lock;
+    Drain drain{c.st};
     Ring r;
     const bool staged = begin(c, s, n, r, lock);
     const int total = (int)r.chunks.size();
@@ -177,6 +189,7 @@ void copy_to_device(Ctx& c, const CopySegment* s, int n, bool wait) {
         if (wait) FOPIS_CUDA(cudaStreamSynchronize(c.st));
         return;
     }
+    drain.staged = true;
     for (int i = 0; i < total; ++i) {
         r.wait_done(i);
         const Chunk& k = r.chunks[i];
@@ -188,6 +201,7 @@ void copy_to_device(Ctx& c, const CopySegment* s, int n, bool wait) {
             r.open.store(back + kSlots + 1, std::memory_order_release);
         }
     }
+    drain.staged = false;
     FOPIS_CUDA(cudaStreamSynchronize(c.st));   // the slots are free for the next copy
 }
 
