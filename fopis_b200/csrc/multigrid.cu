@@ -177,31 +177,13 @@ __global__ void __launch_bounds__(kMarchX * kMarchY) residual_march_kernel(Lv L)
     }
 }
 
-// The first red half sweep from u = 0, which also zeroes the black nodes: red
-// nodes get omega (f/scale) / 6 (their neighbours are all zero).
-template <int A>
-__global__ void __launch_bounds__(kMarchX * kMarchY) rb_first_march_kernel(Lv L) {
-    pdl_entry();
-    const int c = blockIdx.x * kMarchX + threadIdx.x;
-    const int b = blockIdx.y * kMarchY + threadIdx.y;
-    const int a0 = blockIdx.z * A;
-    if (b >= L.n1 || c >= L.n2) return;
-#pragma unroll
-    for (int e = 0; e < A; ++e) {
-        const int a = a0 + e;
-        if (a >= L.n0) break;
-        const long long at = ((long long)a * L.n1 + b) * L.n2 + c;
-        L.u[at] = ((a + b + c) & 1) ? 0.0f : kOmega * (L.f[at] * L.inv_scale) * (1.0f / 6.0f);
-    }
-}
-
-// Red value of the first half sweep from u = 0 (rb_first_march_kernel's formula).
+// Red value of the first half sweep from u = 0: omega (f/scale) / 6 (the neighbours are all zero).
 __device__ __forceinline__ float red_from_zero(float f, float inv_scale) {
     return kOmega * (f * inv_scale) * (1.0f / 6.0f);
 }
 
 // The first full red-black sweep from u = 0 in one pass: red nodes as
-// rb_first_march_kernel sets them, black nodes as rb_march_kernel's black half
+// red_from_zero gives them, black nodes as rb_march_kernel's black half
 // sweep then updates them, with the six red neighbours evaluated from f in
 // place (on red-black levels every neighbour of a black node is red). The
 // additions run in march_nsum's order, so the values equal the two passes'.
