@@ -116,3 +116,26 @@ def test_near_uniform_periodic_charge(gpu_available, nxyz):
             most = tol * np.linalg.norm(f - f.mean()) + (2.0 ** -53 * abs(f.mean()) + 24 * 2.0 ** -53 * np.abs(phi).max()) * np.sqrt(f.size)
             assert np.linalg.norm(r - r.mean()) <= most
     g.close()
+
+
+@pytest.mark.parametrize("nxyz,boundary,cap", [
+    ((33, 34, 35), "DDDDDD", 100), ((20, 19, 18), "PPPPPP", 100), ((66, 35, 34), "DDPPNN", 100), ((24, 24, 24), "PPPPPP", 1),
+    ((515, 66, 65), "DDDDDD", 100)])
+def test_host_driven_loop_gives_the_same(gpu_available, monkeypatch, nxyz, boundary, cap):
+    """FOPIS_SOLVE_HOST_LOOP=1 runs the same kernels with the host deciding: the same potential bit for bit, the same
+    counts and residuals, the hand-over from diverging V-cycles included."""
+    dx, dt = plasma_units()
+    sp = [SpeciesInfo("Electron", "ambient", 1.0, -1.0, 1e7, 1.0, 1)]
+    p, norm = make_params(nxyz, boundary, dx, dt, sp, tol=1e-12, guess=_abi.GUESS_ZERO, max_vcycles=cap)
+    rho = np.random.default_rng(8).standard_normal(tuple(n + 2 for n in nxyz)) * 1e6 + 3e5
+    got = []
+    for env in ("0", "1"):
+        monkeypatch.setenv("FOPIS_SOLVE_HOST_LOOP", env)
+        g = RootGrid(config.SimConfig(params=p, norm=norm, species=sp))
+        g.set_field(_abi.FIELD_RHO0, rho)
+        rc = g.solvePoisson()
+        st = g.stats()
+        got.append((rc, st.converged, st.vcycles_last, st.residual_last, st.residual_initial, g.getPhi()))
+        g.close()
+    assert got[0][0] == (0 if cap > 1 else _abi.ERR_NOT_CONVERGED)
+    assert got[0][:5] == got[1][:5] and np.array_equal(got[0][5], got[1][5])
