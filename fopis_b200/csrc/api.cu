@@ -388,7 +388,7 @@ int fopis_create(const fopis_params* p, int device, void** out) {
         if (p->solver == FOPIS_SOLVER_EM) em_alloc(x);
         mg_setup(x);
         mg_prepare(x);
-        FOPIS_CUDA(cudaDeviceSynchronize());
+        settle_uploads(x);
         return FOPIS_OK;
     });
     if (rc != FOPIS_OK) {

@@ -351,6 +351,14 @@ void launch_absorb(Ctx& c);
 void launch_secondary(Ctx& c, bool fused);   // emission of the pending incidents' secondaries
 void launch_energy(Ctx& c);
 void sync_scalars(Ctx& c);
+// Waits for what set-up put on the legacy stream (plain copies and fills), before
+// kernels of c.st read it, and for c.st. Not cudaDeviceSynchronize, which fails
+// while another thread's context records its solve graph, and breaks that
+// recording.
+inline void settle_uploads(Ctx& c) {
+    FOPIS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+    FOPIS_CUDA(cudaStreamSynchronize(c.st));
+}
 // hostcopy.cu
 struct CopySegment {
     void* dev;

@@ -1461,7 +1461,7 @@ static bool mg_to_direct(Ctx& c) {
     try {
         direct_setup(c.dir, c.mg[0].n, c.mg[0].per);
         FOPIS_CUDA(cudaMalloc(&partials, sizeof(double) * kDirectPartials * blocks));
-        FOPIS_CUDA(cudaDeviceSynchronize());   // the tables are there before c.st reads them
+        settle_uploads(c);
     } catch (const CudaError& e) {
         cudaGetLastError();
         direct_free(c.dir);
