@@ -507,7 +507,7 @@ int fopis_get_charge_map(void* h, int id, double* out, int n) {
 int fopis_set_charge_map(void* h, int id, const double* in, int n) {
     return guarded(h, [&](Ctx& c) -> int {
         if (id < 0 || id >= (int)c.objs.size() || !in || n != c.nsp * c.objs[id].n) throw ApiError{FOPIS_ERR_ARG, "object id or size"};
-        FOPIS_CUDA(cudaMemcpy(c.objs[id].charge_map, in, sizeof(double) * n, cudaMemcpyHostToDevice));
+        copy_to_device(c, c.objs[id].charge_map, in, sizeof(double) * n);
         return FOPIS_OK;
     });
 }
@@ -559,13 +559,13 @@ int fopis_set_incidents(void* h, const double* in, int64_t n) {
         double* dst[7] = {c.inc.trem, c.inc.x, c.inc.y, c.inc.z, c.inc.vx, c.inc.vy, c.inc.vz};
         if (n > 0) {
             for (int q = 0; q < 7; ++q)
-                FOPIS_CUDA(cudaMemcpy(dst[q], col[q].data(), sizeof(double) * n, cudaMemcpyHostToDevice));
-            FOPIS_CUDA(cudaMemcpy(c.inc.object, ob.data(), n, cudaMemcpyHostToDevice));
-            FOPIS_CUDA(cudaMemcpy(c.inc.species, sp.data(), n, cudaMemcpyHostToDevice));
-            FOPIS_CUDA(cudaMemcpy(c.inc.axis, ax.data(), n, cudaMemcpyHostToDevice));
+                copy_to_device(c, dst[q], col[q].data(), sizeof(double) * n);
+            copy_to_device(c, c.inc.object, ob.data(), n);
+            copy_to_device(c, c.inc.species, sp.data(), n);
+            copy_to_device(c, c.inc.axis, ax.data(), n);
         }
         const unsigned long long nn = (unsigned long long)n;
-        FOPIS_CUDA(cudaMemcpy(&c.d_sc->incident_n, &nn, sizeof(nn), cudaMemcpyHostToDevice));
+        copy_to_device(c, &c.d_sc->incident_n, &nn, sizeof(nn));
         return FOPIS_OK;
     });
 }

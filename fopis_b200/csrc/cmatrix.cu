@@ -434,19 +434,19 @@ void object_upload(Ctx& c, ObjectDev& o, const fopis_object_desc* d, int id) {
     copy_to_device(c, c.cellmap, cmap.data(), c.N);
     mark_brick_bodies(c);
     FOPIS_CUDA(cudaMalloc(&o.nodes, sizeof(int32_t) * o.n));
-    FOPIS_CUDA(cudaMemcpy(o.nodes, lin.data(), sizeof(int32_t) * o.n, cudaMemcpyHostToDevice));
+    copy_to_device(c, o.nodes, lin.data(), sizeof(int32_t) * o.n);
     FOPIS_CUDA(cudaMalloc(&o.C, sizeof(double) * (size_t)o.n * o.n));
     FOPIS_CUDA(cudaMalloc(&o.colsum, sizeof(double) * o.n));
     FOPIS_CUDA(cudaMalloc(&o.charge_tmp, sizeof(long long) * (size_t)c.nsp * o.n));
     FOPIS_CUDA(cudaMalloc(&o.charge_map, sizeof(double) * (size_t)c.nsp * o.n));
     FOPIS_CUDA(cudaMalloc(&o.phis, sizeof(double) * o.n));
     FOPIS_CUDA(cudaMalloc(&o.drho_buf, sizeof(double) * 3 * o.n));
-    FOPIS_CUDA(cudaMemset(o.drho_buf, 0, sizeof(double) * 3 * o.n));
+    FOPIS_CUDA(cudaMemsetAsync(o.drho_buf, 0, sizeof(double) * 3 * o.n, c.st));
     for (int q = 0; q < 3; ++q) o.drho[q] = o.drho_buf + (size_t)q * o.n;
     FOPIS_CUDA(cudaMalloc(&o.scal, sizeof(double) * 8));
-    FOPIS_CUDA(cudaMemset(o.charge_tmp, 0, sizeof(long long) * (size_t)c.nsp * o.n));
-    FOPIS_CUDA(cudaMemset(o.charge_map, 0, sizeof(double) * (size_t)c.nsp * o.n));
-    FOPIS_CUDA(cudaMemset(o.scal, 0, sizeof(double) * 8));
+    FOPIS_CUDA(cudaMemsetAsync(o.charge_tmp, 0, sizeof(long long) * (size_t)c.nsp * o.n, c.st));
+    FOPIS_CUDA(cudaMemsetAsync(o.charge_map, 0, sizeof(double) * (size_t)c.nsp * o.n, c.st));
+    FOPIS_CUDA(cudaMemsetAsync(o.scal, 0, sizeof(double) * 8, c.st));
     o.is_fixed = d->is_potential_fixed;
     o.fixed_potential = d->fixed_potential;
     o.offset = d->initial_potential_offset;
@@ -471,7 +471,7 @@ void object_upload(Ctx& c, ObjectDev& o, const fopis_object_desc* d, int id) {
     if (o.dielectric) {
         if (!d->capacitance) throw ApiError{FOPIS_ERR_ARG, "a dielectric surface needs its node capacitances"};
         FOPIS_CUDA(cudaMalloc(&o.capacitance, sizeof(double) * o.n));
-        FOPIS_CUDA(cudaMemcpy(o.capacitance, d->capacitance, sizeof(double) * o.n, cudaMemcpyHostToDevice));
+        copy_to_device(c, o.capacitance, d->capacitance, sizeof(double) * o.n);
     }
     // lit nodes of the emitting face (Spacecraft::emitParticles, Spacecraft.cpp:836-886)
     std::vector<int32_t> lit, lit_ijk;
@@ -493,8 +493,8 @@ void object_upload(Ctx& c, ObjectDev& o, const fopis_object_desc* d, int id) {
     o.n_lit = (int)lit.size();
     if (o.n_lit) {
         FOPIS_CUDA(cudaMalloc(&o.lit, sizeof(int32_t) * 2 * o.n_lit));
-        FOPIS_CUDA(cudaMemcpy(o.lit, lit.data(), sizeof(int32_t) * o.n_lit, cudaMemcpyHostToDevice));
-        FOPIS_CUDA(cudaMemcpy(o.lit + o.n_lit, lit_ijk.data(), sizeof(int32_t) * o.n_lit, cudaMemcpyHostToDevice));
+        copy_to_device(c, o.lit, lit.data(), sizeof(int32_t) * o.n_lit);
+        copy_to_device(c, o.lit + o.n_lit, lit_ijk.data(), sizeof(int32_t) * o.n_lit);
     }
 }
 

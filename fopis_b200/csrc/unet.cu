@@ -547,7 +547,6 @@ __global__ void __launch_bounds__(256) feat_write_kernel(FeatArgs F, const doubl
     }
 }
 
-// phi += sigma_d * prediction on the unknowns.
 // The predicted increment in the glue layout (FP64), zero off the unknowns.
 __global__ void __launch_bounds__(256) predict_kernel(FeatArgs F, const float* out, const double* stats, int cx,
                                                       double* pred) {
@@ -559,6 +558,7 @@ __global__ void __launch_bounds__(256) predict_kernel(FeatArgs F, const float* o
     }
 }
 
+// phi += sigma_d * prediction on the unknowns.
 __global__ void __launch_bounds__(256) apply_guess_kernel(FeatArgs F, const float* out, const double* stats,
                                                           double* phi) {
     const double sd = stats[7];
@@ -1035,7 +1035,7 @@ void check_err(Ctx& c, Net& n) {
                                                 std::to_string(e) + ")"};
 }
 
-void init_params(const Ctx& c, Net& n) {
+void init_params(Ctx& c, Net& n) {
     std::vector<float> h(n.nprm, 0.0f);
     const uint64_t seed = c.p.seed ^ 0x5eedu;
     uint32_t ctr = 0;
@@ -1049,7 +1049,7 @@ void init_params(const Ctx& c, Net& n) {
         for (long long i = 0; i < 27LL * d.cout * d.cin; ++i) h[d.w_off + i] = (float)(sd * normal());
     }
     for (int ch = 0; ch < kHead; ++ch) h[n.T.head_off + ch] = (float)(0.05 * normal());
-    FOPIS_CUDA(cudaMemcpy(n.prm, h.data(), sizeof(float) * n.nprm, cudaMemcpyHostToDevice));
+    copy_to_device(c, n.prm, h.data(), sizeof(float) * n.nprm);
 }
 
 }  // namespace
@@ -1083,10 +1083,10 @@ Net* create(Ctx& c) {
             t.level = kSlot[s].level;
             t.g = &n->G[t.level];
             FOPIS_CUDA(cudaMalloc(&t.base, t.bytes()));
-            FOPIS_CUDA(cudaMemset(t.base, 0, t.bytes()));
+            FOPIS_CUDA(cudaMemsetAsync(t.base, 0, t.bytes(), c.st));
         }
         FOPIS_CUDA(cudaMalloc(&n->out, sizeof(float) * n->G[0].P));
-        FOPIS_CUDA(cudaMemset(n->out, 0, sizeof(float) * n->G[0].P));
+        FOPIS_CUDA(cudaMemsetAsync(n->out, 0, sizeof(float) * n->G[0].P, c.st));
         long long off = 0, img = 0;
         for (int l = 0; l < kLayers; ++l) {
             LayerDesc& d = n->T.l[l];
@@ -1108,17 +1108,17 @@ Net* create(Ctx& c) {
         FOPIS_CUDA(cudaMalloc(&n->grad, sizeof(float) * off));
         FOPIS_CUDA(cudaMalloc(&n->m1, sizeof(float) * off));
         FOPIS_CUDA(cudaMalloc(&n->m2, sizeof(float) * off));
-        FOPIS_CUDA(cudaMemset(n->grad, 0, sizeof(float) * off));
-        FOPIS_CUDA(cudaMemset(n->m1, 0, sizeof(float) * off));
-        FOPIS_CUDA(cudaMemset(n->m2, 0, sizeof(float) * off));
+        FOPIS_CUDA(cudaMemsetAsync(n->grad, 0, sizeof(float) * off, c.st));
+        FOPIS_CUDA(cudaMemsetAsync(n->m1, 0, sizeof(float) * off, c.st));
+        FOPIS_CUDA(cudaMemsetAsync(n->m2, 0, sizeof(float) * off, c.st));
         FOPIS_CUDA(cudaMalloc(&n->img, sizeof(bf16) * img));
         FOPIS_CUDA(cudaMalloc(&n->stats, 16 * sizeof(double)));
-        FOPIS_CUDA(cudaMemset(n->stats, 0, 16 * sizeof(double)));
+        FOPIS_CUDA(cudaMemsetAsync(n->stats, 0, 16 * sizeof(double), c.st));
         FOPIS_CUDA(cudaMallocHost(&n->h_stats, 16 * sizeof(double)));
         std::memset(n->h_stats, 0, 16 * sizeof(double));
         for (auto& e : n->ev) FOPIS_CUDA(cudaEventCreate(&e));
         FOPIS_CUDA(cudaMalloc(&n->err, sizeof(unsigned int)));
-        FOPIS_CUDA(cudaMemset(n->err, 0, sizeof(unsigned int)));
+        FOPIS_CUDA(cudaMemsetAsync(n->err, 0, sizeof(unsigned int), c.st));
         init_params(c, *n);
     } catch (...) {
         unet_free(c);
