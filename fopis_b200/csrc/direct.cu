@@ -626,7 +626,8 @@ void direct_setup(DirectShape& S, const int n[3], const int per[3]) {
     // the attribute belongs to the function, which contexts of other sizes share
     allow_tile<64>();
     allow_tile<32>();
-    allow_tile<16>();
+    for (const auto& x : S.ax)
+        if (tile_smem(x, 32 + 4) > kMostSmem) { allow_tile<16>(); break; }
 }
 
 void direct_free(DirectShape& S) {
