@@ -2,7 +2,7 @@
 """Benchmark of the FOPIS electrostatic PIC timestep on B200.
 
 Metric: particle-steps/s of RootGrid::mainLoopES (one step = push + gather +
-boundaries + absorption + deposit + emission + injection + two multigrid
+boundaries + absorption + deposit + emission + injection + two
 Poisson solves with the capacity-matrix correction + E field + periodic sort)
 on the 128^3-cell workload: Dirichlet box with thermal injection through all
 six faces, electrons + ions (mass ratio 100) at 32 particles/cell/species, a
@@ -196,9 +196,9 @@ WORKLOADS = {
 def workload_desc(name: str, ppc) -> str:
     text, default_ppc = WORKLOADS[name]
     if name == "em128":
-        return f"{name}: {text}, {ppc or default_ppc} ppc/species, one Poisson solve at start-up (MG to 1e-8)"
+        return f"{name}: {text}, {ppc or default_ppc} ppc/species, one Poisson solve at start-up (to 1e-8)"
     solves = "1 solve/step" if name == "periodic32" else "2 solves/step"
-    return f"{name}: {text}, {ppc or default_ppc} ppc/species, MG to ||r||/||f|| <= 1e-8, {solves}"
+    return f"{name}: {text}, {ppc or default_ppc} ppc/species, Poisson to ||r||/||f|| <= 1e-8, {solves}"
 
 
 def barrier(world: int):
@@ -634,8 +634,8 @@ def main():
     hbm, peak_kind = peaks()
     base = {"metric": "particle-steps/s", "unit": "particle-steps/s", "n_gpus": world, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "data": "synthetic (Philox-seeded Maxwellian plasma)",
-            "dtype": ("fp32 particles, int64 fixed-point rho, fp32 smoother in fp64 refinement" if args.precision == "mixed"
-                      else "fp64 particles, fp64 deposit, fp32 smoother in fp64 refinement"),
+            "dtype": ("fp32 particles, int64 fixed-point rho, fp32 corrections in fp64 refinement" if args.precision == "mixed"
+                      else "fp64 particles, fp64 deposit, fp32 corrections in fp64 refinement"),
             # the same dict on both arms: what is run, not how each arm runs it
             "config": {"workload": workload_desc(args.workload, args.ppc),
                        "parallelism": f"replicas x{world}", "sort_interval": args.sort_interval}}

@@ -6,9 +6,11 @@
 // basis of its axis: sines between held faces, the real Fourier basis on a
 // periodic axis. e = Q (Q^T r) / (lambda_a + lambda_b + lambda_c), one
 // transform per axis and direction, any axis length, so a correction is exact
-// up to FP32 rounding: it lowers ||r|| by 1e-4 (smooth r) to 1e-6 (noise),
-// where a V(2,1) multigrid cycle lowers it by 0.18 and, on an axis whose length
-// stops coarsening early (an odd periodic one), hardly at all. The residual
+// up to FP32 rounding: it lowers ||r|| to 1e-6 of it where r is noise (7e-7 at
+// 63^3, 3e-6 at 255^3) and to 1e-4 where r is smooth (9e-5 and 2e-3, the rounding of
+// the large e), where a V(2,1) multigrid cycle lowers it to 0.18 and, on an axis
+// whose length stops coarsening early (an odd periodic one) or halves evenly between
+// held faces, less or not at all. The residual
 // stays FP64 and decides, as in the multigrid refinement.
 //
 // Transforms are dense products with the basis, halved by its parity: index
@@ -25,9 +27,11 @@
 // multiply-adds keep both pipes even. The matrices arrive in chunks of 16 rows
 // through a three-stage cp.async ring whose first stages are requested before
 // the wait for the previous kernel. At 127^3 a transform takes 16 us, at 255^3
-// 156 us (27 TFLOP/s of the 72 that FP32 multiply-adds reach here; bound by
-// the instructions around them and, at 127^3, by the load and store phases of
-// the 1.7 tiles an SM gets). 4 x 4 tiles of both halves: 22 us at 127^3.
+// 156 us (27 TFLOP/s of the 72 that FP32 multiply-adds reach here). There the FP32
+// pipe is busy 47-49 % of the time and the issue slots 44 %: shared memory leaves
+// room for one CTA, two warps a scheduler, which do not cover the waits on each
+// other's results; at 127^3 the load and store phases of the 1.7 tiles an SM gets
+// come on top. 4 x 4 tiles of both halves: 22 us at 127^3.
 #include "direct.cuh"
 
 #include <algorithm>
@@ -41,9 +45,11 @@ namespace {
 // Unknowns per axis. A correction costs O(n^4), a V-cycle O(n^3), but a solve
 // takes 2 of the first where it takes 7-8 of the second; cold solves to 1e-8,
 // six held faces, V-cycles against this: 127^3 1.31 / 0.26 ms, 255^3 6.9 / 2.3,
-// 383^3 20.9 / 13.9, 511^3 48.2 / 32.6. 120 x 75 x 50 with two periodic axes
-// (coarsening stops at 60 x 37 x 25): 65 / 0.3 ms. Beyond, a tile of 32 lines
-// soon outgrows shared memory as the lead shrinks.
+// 383^3 20.9 / 13.9, 511^3 48.2 / 32.6, 575^3 57.5 / 62.7, 639^3 77.7 / 87.3,
+// 767^3 133 / 273. 120 x 75 x 50 with two periodic axes (coarsening stops at 60 x 36
+// x 25): 65 / 0.3 ms. So the line is where cubes cross over. It looks at the longest
+// axis alone: a long thin box beyond it would still gain (513 x 18 x 18 61 / 0.4 ms,
+// 767 x 63 x 63 13 / 1.0, 639 x 319 x 319 20.8 / 16.8).
 constexpr int kDirectMax = 512;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;

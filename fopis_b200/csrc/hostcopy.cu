@@ -2,7 +2,7 @@
 //
 // cudaMemcpy stages pageable memory through one thread: 4.2 GB/s into freshly
 // allocated pages (that thread takes every page fault), 9 GB/s out of them,
-// where the link carries 50. Here chunks go through a ring of pinned slots, the
+// where the link carries 54. Here chunks go through a ring of pinned slots, the
 // calling thread issuing the device copies and a few threads copying between
 // the slots and the caller's memory, so faults and memory copies run in
 // parallel and beside the link. A potential of 139 MB into a new array: 33 ->
@@ -28,9 +28,10 @@ namespace {
 
 constexpr size_t kSlot = 512 * 1024;
 constexpr int kSlots = 16;
-// Below this an allocator hands out pages that are mapped already, where
-// cudaMemcpy moves 17 GB/s and the threads are no faster (18 MB: 1.0 against
-// 1.6 ms); above it every allocation is new pages.
+// Below this an allocator that has freed such a block before hands out pages that
+// are mapped already, where cudaMemcpy moves 18-20 GB/s and the threads, started for
+// each copy, are no faster (18 MB: 1.0 against 1.6 ms); above it every allocation is
+// new pages. (A first read of a smaller field pays its page faults here too.)
 constexpr size_t kStaged = 32 << 20;
 
 std::mutex g_ring_mutex;

@@ -1097,8 +1097,8 @@ __global__ void __launch_bounds__(kBrickThreads, 4) push_brick_kernel(PushArgs a
 // at 32^3 once electrons move 0.35 cells a step).
 // Warp sums and 64-bit global atomics for every particle (em_warp_move_current)
 // took 11.0 ms at 128^3 (1.34e8 particles), this 6.15 (1.2 TB/s of the 56 B a
-// particle); it is bound by the shared-memory and gather wavefronts (69 % of
-// the LSU data path busy) and the latency of the gather. One low word with a
+// particle); it is bound by the shared-memory and gather wavefronts (63 and 70 %
+// of the LSU data path's for ions and electrons at 64^3) and the latency of the gather. One low word with a
 // carry instead of two pieces: 0.25 ms more. 512 threads, because the tile and the batch
 // leave room for two CTAs per SM.
 constexpr int kEmThreads = 512;

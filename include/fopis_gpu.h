@@ -90,7 +90,7 @@ typedef struct fopis_species {
 
 typedef enum fopis_precision {
     FOPIS_MIXED = 0,   /* int32 cell + FP32 offset/velocity particles, int64 fixed-point rho,
-                          FP32 smoother inside FP64 iterative refinement */
+                          FP32 corrections inside FP64 iterative refinement */
     FOPIS_FP64 = 1     /* int32 cell + FP64 offset/velocity particles, FP64 E gather and push,
                           FP64 CIC deposit (atomic sums), phi from the same FP64 residual
                           refinement to the requested tolerance; the reference run for
@@ -118,7 +118,8 @@ typedef struct fopis_params {
     int nspecies;                /* Environment::num_of_particle_types; order ambient -> photo */
     fopis_species species[FOPIS_MAX_SPECIES];
     double poisson_tol;          /* ||f - A phi||_2 <= tol ||f||_2 ; 0 -> 1e-8 */
-    int max_vcycles;             /* cap on corrections (V-cycles) per solve; 0 -> 100 */
+    int max_vcycles;             /* cap on corrections (V-cycles; then again on the direct
+                                    corrections, where these take over) per solve; 0 -> 100 */
     int guess_mode;              /* fopis_guess_mode */
     int sort_interval;           /* counting-sort period in steps; 0 -> 8 */
     int remove_interval;         /* removeInvalidParticles period (RootGrid.cpp:136-140); 0 -> 50 */
@@ -207,7 +208,7 @@ typedef struct fopis_stats {
                                     it), emit, position with the currents + inject, 0, rho, E update,
                                     B update, sort */
     int64_t kernel_launches;     /* kernels this context has launched since creation */
-    int solve_mode;              /* 0: host-driven V-cycle loop; 1: one CUDA graph with a device-side
+    int solve_mode;              /* 0: host-driven loop of corrections; 1: one CUDA graph with a device-side
                                     loop; 2: the same graph with programmatic dependent launches */
     int pad;
     double residual_pointwise;   /* last solve, RootGrid::checkPhiResidual's measure

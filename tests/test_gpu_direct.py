@@ -4,8 +4,9 @@ periodic axes, axes around the multiples of the 8 modes, 16 matrix rows, 64
 lines and 128-mode passes it works in, and axes beyond its limit, which the
 multigrid cycle takes as long as it converges: where halved even counts make it
 diverge, the direct correction takes over, in the EM mode as well. The residual of the returned potential, formed here in
-FP64, has to meet the tolerance the solve reports; a correction lowers it by
-more than 1e-3, so two or three suffice for 1e-10 on any shape."""
+FP64, has to meet the tolerance the solve reports; a correction lowers it to 1e-3
+or less at these sizes, and what it leaves is noise, which the next lowers to 1e-5
+or less, so two or three suffice for 1e-10."""
 import numpy as np
 import pytest
 
