@@ -425,18 +425,19 @@ __device__ ResidualSums block_sums(ResidualSums s, bool allper) {
 // the graph's loop takes another correction (tolerance not met, cap not
 // reached, residual finite). In an all-periodic box the mean of f, subtracted as a
 // rounded number, leaves a constant of a rounding or so in f and in every r, which
-// no phi can lower: it is taken out of both norms (M: the unknowns' number). And
-// charge that differs from its mean by less than a rounding of the mean over the
-// tolerance (1e-8 of it at 1e-8) is solved to that rounding instead: fm carries it.
-__device__ void decide(const DirectStep& d, const ResidualSums& t, double M, double fm) {
+// no phi can lower: it is taken out of both norms. And charge that differs from its
+// mean by less than a rounding of the mean over the tolerance (1e-8 of it at 1e-8)
+// is solved to that rounding instead: fm carries it.
+__device__ void decide(const DirectStep& d, const DirectOuter& O, const ResidualSums& t, double fm) {
     double* red = d.sc->red;
-    const double constant = t.rsum * (t.rsum / M);
+    const double constant = O.allper ? t.rsum * t.rsum * O.inv_m : 0.0;
     const double r2 = t.r2 >= constant ? t.r2 - constant : (isfinite(t.r2) ? 0.0 : t.r2), worst = t.worst;
     const double res = sqrt(r2);
     if (d.mode & DIRECT_START) {
         red[6] = d.host->red[6];
         red[7] = d.host->red[7];
-        double fn = fmax(sqrt(fmax(t.f2 - constant, 0.0)), 0x1p-53 * fabs(fm) * sqrt(M) / red[6]);
+        double fn = sqrt(fmax(t.f2 - constant, 0.0));
+        if (O.allper) fn = fmax(fn, 0x1p-53 * fabs(fm) * O.root_m / red[6]);
         red[5] = fn > 0.0 ? fn : 1.0;
         red[8] = 0.0;
         red[9] = res;
@@ -522,7 +523,7 @@ __global__ void __launch_bounds__(kThreads) direct_residual_kernel(DirectShape S
     }
     t = block_sums(t, O.allper);
     if (threadIdx.x != 0) return;
-    decide(step, t, (double)S.n0 * S.n1 * S.n2, fm);
+    decide(step, O, t, fm);
 }
 
 size_t ring_smem(const DirectAxis& x) { return sizeof(float) * kStages * 2 * kRows * pass_modes(x.hp); }

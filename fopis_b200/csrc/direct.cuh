@@ -15,6 +15,7 @@ struct DirectOuter {
     int per[3], nref[3];  // periodic axes and their node counts
     int allper;
     double eps0, inv_eps0;
+    double inv_m, root_m;   // of the unknowns' number m: 1 / m and its square root
 };
 
 // What the residual kernel's last block does with the sums: keep them (the

@@ -1493,6 +1493,9 @@ static DirectOuter direct_outer(const Ctx& c) {
     d.allper = O.p0 && O.p1 && O.p2;
     d.eps0 = c.p.eps0;
     d.inv_eps0 = O.inv_eps0;
+    const double m = (double)O.n0 * O.n1 * O.n2;
+    d.inv_m = 1.0 / m;
+    d.root_m = std::sqrt(m);
     return d;
 }
 
