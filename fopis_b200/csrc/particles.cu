@@ -1112,6 +1112,7 @@ struct EmTile {
     float o[3][kBatchPad], v[3][kBatchPad];              // start offsets and velocity
     unsigned cells[kBatchPad];                           // start cell of a move that stays; else none, new and old cell, 10 bits each
     int was[kBatchPad], now[kBatchPad];                  // strays: packed cells, now -1 once gone, kDeposits if it deposits
+                                                         // outside the window (one back inside has its batch entry)
     unsigned short list[kBatch];                         // entries that change their cell from the front, strays from the back
     int listed[2], strays[2];                            // of this batch and the next
 };
@@ -1284,7 +1285,7 @@ __global__ void __launch_bounds__(kEmThreads, 2) em_brick_kernel(PushArgs a, con
                     if (had && !tiled) {
                         T.list[kBatch - 1 - (at + __popc(n & ((1u << lane) - 1u)))] = (unsigned short)e;
                         T.was[e] = cell;
-                        T.now[e] = moved ? pack_cell(st.i, st.j, st.k) | (live ? kDeposits : 0) : -1;
+                        T.now[e] = moved ? pack_cell(st.i, st.j, st.k) | (live && !inwin ? kDeposits : 0) : -1;
                     }
                 }
                 const unsigned qa = (unsigned)__float2int_rn(st.ox * kDepositScale);

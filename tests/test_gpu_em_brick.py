@@ -73,8 +73,10 @@ def test_currents_and_charge_match_fp64(gpu_available, n, boundary, per_cell, sp
 @pytest.mark.parametrize("n,boundary,per_cell,speed,steps,lo,hi", [
     (5, "PPPPPP", 6, 0.3, 1, (0, 0, 0), None), (9, "DDDDDD", 8, 0.05, 1, (0, 0, 0), None),
     (13, "PPDDPP", 4, 0.6, 1, (0, 0, 0), None), (18, "DDDDDD", 3, 0.3, 3, (0, 0, 0), None),
-    (11, "PPPPPP", 12, 0.2, 1, (0, 0, 0), (1, 1, 1)), (13, "DDDDDD", 5, 0.3, 2, (3, 7, 8), (4, 8, 9))])
+    (11, "PPPPPP", 12, 0.2, 1, (0, 0, 0), (1, 1, 1)), (13, "DDDDDD", 5, 0.3, 2, (3, 7, 8), (4, 8, 9)),
+    (4, "PPPPPP", 12, 0.3, 14, (0, 0, 0), None), (9, "PPPPPP", 6, 0.6, 20, (0, 0, 0), None)])
 def test_charge_matches_replay(gpu_available, n, boundary, per_cell, speed, steps, lo, hi):
+    """The last two: particles that leave their brick's window and come back into it, around the box, between sorts."""
     g, _, _, _ = start(n, boundary, _abi.MIXED, per_cell, speed, lo, hi)
     for _ in range(steps):
         assert g.mainLoopEM(1) == 0
