@@ -46,7 +46,9 @@ namespace {
 // takes 2 of the first where it takes 7-8 of the second; cold solves to 1e-8,
 // six held faces, V-cycles against this: 127^3 1.31 / 0.26 ms, 255^3 6.9 / 2.3,
 // 383^3 20.9 / 13.9, 511^3 48.2 / 32.6, 575^3 57.5 / 62.7, 639^3 77.7 / 87.3,
-// 767^3 133 / 273. 120 x 75 x 50 with two periodic axes (coarsening stops at 60 x 36
+// 767^3 133 / 273. (From a start within 1e-6, 2 V-cycles against one correction,
+// cubes cross earlier: 383^3 5.5 / 7.1, 511^3 12.3 / 16.7; within 1e-3, 4 against one,
+// where they do cold.) 120 x 75 x 50 with two periodic axes (coarsening stops at 60 x 36
 // x 25): 65 / 0.3 ms. So the line is where cubes cross over. It looks at the longest
 // axis alone: a long thin box beyond it would still gain (513 x 18 x 18 61 / 0.4 ms,
 // 767 x 63 x 63 13 / 1.0, 639 x 319 x 319 20.8 / 16.8).
