@@ -85,14 +85,20 @@ __device__ __forceinline__ bool axis_boundary_d(const Grid& g, int axis, double&
     return true;
 }
 
-// Split an FP64 coordinate into node cell index and in-cell offset (FP32 in
-// the mixed mode, where rounding can reach 1 and carries into the cell).
+// Split an FP64 coordinate of an axis into node cell index and in-cell offset
+// (FP32 in the mixed mode, where rounding can reach 1 and carries into the cell;
+// a coordinate that rounds up to the length n of a periodic axis is at 0, as the
+// boundary rule has it for x >= n: cell n + 1 would lie beyond the arrays).
 template <typename T>
-__device__ __forceinline__ void split(double x, int& ci, T& o) {
+__device__ __forceinline__ void split(const Grid& g, int axis, double x, int& ci, T& o) {
     const double f = floor(x);
     ci = (int)f + 1;
     o = (T)(x - f);
-    if (o >= (T)1) { o = (T)0; ci += 1; }
+    if (o >= (T)1) {
+        o = (T)0;
+        ci += 1;
+        if (ci == g.n[axis] + 1 && g.per[2 * axis + 1]) ci = 1;
+    }
 }
 
 // FP64 CIC deposit of the FP64 mode: the eight corner weights of a particle
@@ -1401,7 +1407,7 @@ __device__ void finish_source(const SourceArgsT<T>& a, int s, double x, double y
         live = axis_boundary_d(a.g, 0, x) && axis_boundary_d(a.g, 1, y) && axis_boundary_d(a.g, 2, z);
     }
     if (live) {
-        split(x, i, ox); split(y, j, oy); split(z, k, oz);
+        split(a.g, 0, x, i, ox); split(a.g, 1, y, j, oy); split(a.g, 2, z, k, oz);
         if (!cell_in_range(a.g, i, j, k)) { live = false; atomicOr(&a.sc->status, (unsigned)FOPIS_DEV_NONFINITE); }
     }
     bool absorbed = false;
@@ -2004,7 +2010,7 @@ __global__ void ambient_kernel(AmbientArgs<T> a) {
             box_muller(r1.b, r2.a, n0, n1);
             box_muller(r2.b, r3.a, n2, n3);
             vx = a.drift[0] + a.dev * n0; vy = a.drift[1] + a.dev * n1; vz = a.drift[2] + a.dev * n2;
-            split(x, i, ox); split(y, j, oy); split(z, k, oz);
+            split(a.g, 0, x, i, ox); split(a.g, 1, y, j, oy); split(a.g, 2, z, k, oz);
             if (a.cellmap && valid_cell(a.g, i, j, k) && a.cellmap[lin(a.g, i, j, k)]) keep = false;
         }
         const unsigned long long slot = warp_reserve(&a.sc->count[a.s], keep);
@@ -2027,7 +2033,7 @@ __global__ void load56_kernel(SoaT<T> p, long long cap, unsigned long long* coun
         int i = 0, j = 0, k = 0;
         T ox = 0, oy = 0, oz = 0;
         if (keep) {
-            split(in[t].x, i, ox); split(in[t].y, j, oy); split(in[t].z, k, oz);
+            split(g, 0, in[t].x, i, ox); split(g, 1, in[t].y, j, oy); split(g, 2, in[t].z, k, oz);
             if (!cell_in_range(g, i, j, k)) { keep = false; atomicOr(&sc->status, (unsigned)FOPIS_DEV_NONFINITE); }
         }
         const unsigned long long slot = warp_reserve(count, keep);
